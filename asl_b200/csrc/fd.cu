@@ -25,7 +25,10 @@
 #include <nvtx3/nvToolsExt.h>
 #include "aslb.h"
 #include "kernels.h"
+#include "f32x2.cuh"
 #include "lattice.cuh"
+#include "launch.cuh"
+#include "tma.cuh"
 
 namespace aslb {
 namespace {
@@ -99,73 +102,6 @@ __device__ __forceinline__ T fd_cell(CV cvf, UV uvf, EV evf, T D, int cc) {
   return cnew;
 }
 
-// First nonzero component's sign of e_i (pairs i, opp(i) share |q_i|).
-template <int Q>
-__host__ __device__ constexpr int fd_lead_sign(int i) {
-  return FdTemplate<Q>::e(i, 0) != 0 ? FdTemplate<Q>::e(i, 0)
-                                     : (FdTemplate<Q>::e(i, 1) != 0 ? FdTemplate<Q>::e(i, 1) : FdTemplate<Q>::e(i, 2));
-}
-
-// The update without the electric term, regrouped per link i of the
-// template (the same sums as fd_cell, in another order; fewer additions,
-// which the register-blocked kernel needs, while the 2.5-D kernel's d3q7
-// step ran 1.4 % slower with it):
-//   divProduct = sum_i GC_i / 2 (c_i + c_0) (p_i + q_i),
-//   p_i = e_i . u(x + e_i), q_i = e_i . u(x), div(u) = sum_i GC_i p_i,
-// with the laplacian and both sums accumulated per coefficient class (axis,
-// edge or corner vectors) and scaled once; q_i = -q_opp(i) is formed once
-// per pair. cvf(i) = c(x + e_i), uvf(d, i) = u_d(x + e_i).
-template <int Q, class T, bool U, bool CC, class CV, class UV>
-__device__ __forceinline__ T fd_cell_links(CV cvf, UV uvf, T D) {
-  using Tp = FdTemplate<Q>;
-  const T c0 = cvf(0);
-  T q0[3] = {T(0), T(0), T(0)};
-  if constexpr (U) {
-    q0[0] = uvf(0, 0);
-    q0[1] = uvf(1, 0);
-    q0[2] = uvf(2, 0);
-  }
-  T la = T(0), ld = T(0), aa = T(0), ad = T(0), va = T(0), vd = T(0);
-#pragma unroll
-  for (int i = 1; i < Q; ++i) {
-    const T ci = cvf(i);
-    const bool axis = i <= 6, first = i == 1 || i == 7;
-    if (axis) la = first ? ci : la + ci; else ld = first ? ci : ld + ci;
-    if constexpr (U) {
-      // p = e_i . u(x + e_i); q = s e_i . u(x) with s the sign that makes
-      // the leading component positive (the same sum for i and opp(i))
-      const int sg = fd_lead_sign<Q>(i);
-      T p = T(0), qc = T(0);
-      bool fp = true;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const int ed = Tp::e(i, d);
-        if (ed == 0) continue;
-        const T ud = uvf(d, i);
-        p = fp ? (ed > 0 ? ud : -ud) : (ed > 0 ? p + ud : p - ud);
-        qc = fp ? q0[d] : (ed * sg > 0 ? qc + q0[d] : qc - q0[d]);
-        fp = false;
-      }
-      const T pq = sg > 0 ? p + qc : p - qc;
-      const T m = ci + c0;
-      if (axis) aa = first ? m * pq : fma(m, pq, aa); else ad = first ? m * pq : fma(m, pq, ad);
-      if constexpr (CC) {
-        if (axis) va = first ? p : va + p; else vd = first ? p : vd + p;
-      }
-    }
-  }
-  const T lap = T(Tp::lc(0)) * c0 + T(Tp::lc(1)) * la + (Q > 7 ? T(Tp::lc(7)) * ld : T(0));
-  T cnew = D * lap + c0;
-  if constexpr (U) {
-    cnew -= T(0.5 * Tp::gc(1)) * aa + (Q > 7 ? T(0.5 * Tp::gc(7)) * ad : T(0));
-    if constexpr (CC) {
-      cnew /= T(1) - (T(Tp::gc(1)) * va + (Q > 7 ? T(Tp::gc(7)) * vd : T(0)));
-      cnew += lap * (q0[0] * q0[0] + q0[1] * q0[1] + q0[2] * q0[2]) * T(0.5);
-    }
-  }
-  return cnew;
-}
-
 // 2.5-D tiling: a block of 32 x 8 threads owns a 32 (z) x 8 (y) column of
 // cells and walks kFdPlanes x planes, keeping three planes of c (and u) with
 // a one-cell halo in shared memory, so every value is read from HBM about
@@ -185,6 +121,8 @@ __global__ void __launch_bounds__(kFdTZ * kFdTY) k_fd_step(const T* __restrict__
   // three planes of the tile (dynamic: FP64 with velocity and electric fields
   // needs 56 KB)
   extern __shared__ __align__(16) unsigned char fd_smem[];
+  let_next();
+  wait_before();
   auto sm = reinterpret_cast<T(*)[NF][P]>(fd_smem);
   const int tz = threadIdx.x, ty = threadIdx.y, t = ty * kFdTZ + tz;
   const int z0 = blockIdx.x * kFdTZ, y0 = blockIdx.y * kFdTY;  // ghosted origin of the tile
@@ -249,133 +187,241 @@ __global__ void __launch_bounds__(kFdTZ * kFdTY) k_fd_step(const T* __restrict__
   }
 }
 
-// Register-blocked FP32 step (no electric term) for the d3q15 / d3q19
-// templates: a block of 32 (z) x 4 (y) threads owns a 64 x 16 tile of a
-// plane, each thread a 4 x 2 block of cells (two consecutive z, four
-// consecutive y). Three planes of the tile with its one-cell halo sit in a
-// ring of four shared-memory slots; plane x + 2 is loaded into registers
-// during plane x and stored to its slot at the top of the next iteration.
-// The stencil reads of a thread's cells overlap, the unrolled cells read each
-// shared value once, and a thread's two middle columns are one 8-byte load
-// (about 19 shared loads per d3q19 cell instead of 52). The update is
-// fd_cell_links (ASL's sums regrouped per link). Work: the tiles' planes in
-// tile-major order, an equal run of them per resident block (a run that
-// crosses into the next tile restarts the ring there).
-constexpr int kRbTZ = 32;
-
-// The tile and its ring (two resident blocks of 128 threads per SM: eight
-// cells per thread outweigh the lower occupancy; 198 registers). KZ
-// consecutive z cells per thread: with two, a row's columns are shifted by
-// one (column c holds z0 - 1 + c) so each thread's pair sits on an 8-byte
-// boundary and is one shared load.
-struct RbConf {
-  static constexpr int TY = 4, KY = 4, KZ = 2, MINB = 2;
-  static constexpr int CO = KZ == 2 ? 1 : 0;       // column of ghosted z0
-  static constexpr int TZ = kRbTZ * KZ;            // tile cells along z
-  static constexpr int H = TY * KY + 2;            // tile rows with the halo
-  static constexpr int W = TZ + 2 + 2 * CO;        // tile columns with the halo
-  static constexpr int P = H * W;                  // entries of one field plane
-  static constexpr int NT = kRbTZ * TY;            // threads
-  static constexpr int E = (P + NT - 1) / NT;      // entries per thread
-  static constexpr int S = 4;                      // ring slots
-  static_assert(KZ == 1 || KZ == 2, "one or two z cells per thread");
+// FP32 step without the electric term: a block marches along x and reads
+// every plane of its tile once.
+//
+// With e_i, GC_i the template and sum_i GC_i e_i = 0, the product divergence
+//   divProduct = sum_i GC_i / 2 (c_i + c_0) (e_i . u_i + e_i . u_0)
+// is 1/2 [div(c u) + c_0 div(u) + u_0 . grad(c)], so a step needs only linear
+// stencil sums (laplacian and gradient of c, divergences of u and c u), and
+// each plane's contribution to the outputs of the planes before, at and after
+// it is a handful of in-plane sums. A thread owns KY x 2 cells (y, z) of the
+// tile: per plane it reads the KY + 2 rows of its four columns once (two
+// 8-byte shared loads per row and field: the tile's column 0 is the ghosted
+// z0, so they are aligned), forms the sums of its two z cells in packed FP32,
+// finishes the outputs of the previous plane and keeps, for the outputs of
+// the next one, the five sums that its velocity will multiply.
+//
+// The gather over three planes that this replaces read 18.7 shared words per
+// d3q19 cell and was bound by that stream of loads. Planes are staged by
+// 4-byte asynchronous copies (ASL's rows have no alignment) into a ring of
+// three slots, two planes ahead of the arithmetic, without registers.
+// Work: items of `len` planes of a tile, all tiles of an x range before the
+// next range, so that the blocks running together share their tiles' halo
+// rows in L2 (tile by tile, the halos come from HBM again).
+// KY: two, four for d3q7, whose cells carry fewer sums (512x256x256 FP32 with
+// velocity, ms per step with two / four: d3q7 0.187 / 0.183, 0.062 / 0.049 at
+// 256x192x192; d3q19 0.215 / 0.243).
+template <int Q>
+struct MarchConf {
+  static constexpr int KY = Q == 7 ? 4 : 2, TY = 4;  // y cells per thread, warps
+  static constexpr int NT = 32 * TY;            // threads
+  static constexpr int TZ = 64, H = KY * TY + 2, W = TZ + 2, P = H * W;
+  static constexpr int E = (P + NT - 1) / NT;   // staged entries per thread and field
+  static constexpr int S = 3;                   // ring slots
 };
 
-template <bool U>
-constexpr size_t fd_rb_smem() {
-  return (size_t)RbConf::S * (U ? 4 : 1) * RbConf::P * sizeof(float);
+template <int Q, bool U>
+constexpr size_t fd_march_smem() {
+  return (size_t)MarchConf<Q>::S * (U ? 4 : 1) * MarchConf<Q>::P * sizeof(float);
+}
+
+// One row's values at a thread's two cells: the value (m), the sum (s) and
+// the difference (d) of its two z neighbours, of c, u_x, c u_x, u_y, c u_y,
+// u_z, c u_z as far as the sums need them.
+struct MarchRow {
+  F2 cm, cs, cd, um, us, pm, ps, vm, vs, qm, qs, wm, wd, rd;
+};
+
+template <bool U, int P>
+__device__ __forceinline__ MarchRow march_row(const float* b) {
+  auto pair = [](const float* q) {
+    const float2 v = *reinterpret_cast<const float2*>(q);
+    return F2(v.x, v.y);
+  };
+  MarchRow r;
+  const F2 c0 = pair(b), c1 = pair(b + 2);
+  r.cm = F2(c0.hi(), c1.lo());
+  r.cs = add_(c0, c1);
+  r.cd = sub_(c1, c0);
+  if constexpr (U) {
+    const F2 u0 = pair(b + P), u1 = pair(b + P + 2);
+    const F2 v0 = pair(b + 2 * P), v1 = pair(b + 2 * P + 2);
+    const F2 w0 = pair(b + 3 * P), w1 = pair(b + 3 * P + 2);
+    const F2 p0 = mul_(c0, u0), p1 = mul_(c1, u1), q0 = mul_(c0, v0), q1 = mul_(c1, v1);
+    r.um = F2(u0.hi(), u1.lo());
+    r.us = add_(u0, u1);
+    r.pm = F2(p0.hi(), p1.lo());
+    r.ps = add_(p0, p1);
+    r.vm = F2(v0.hi(), v1.lo());
+    r.vs = add_(v0, v1);
+    r.qm = F2(q0.hi(), q1.lo());
+    r.qs = add_(q0, q1);
+    r.wm = F2(w0.hi(), w1.lo());
+    r.wd = sub_(w1, w0);
+    r.rd = sub_(mul_(c1, w1), mul_(c0, w0));
+  }
+  return r;
 }
 
 template <int Q, bool U, bool CC>
-__global__ void __launch_bounds__(RbConf::NT, RbConf::MINB)
-    k_fd_step_rb(const float* __restrict__ c, float* __restrict__ cn, const float* __restrict__ u, FdGrid g,
-                 float D, int ntz, long long units, long long per_block) {
+__global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
+    k_fd_march(const float* __restrict__ c, float* __restrict__ cn, const float* __restrict__ u, FdGrid g, float Df,
+               int ntz, int tiles, int len, int items) {
   using Tp = FdTemplate<Q>;
-  using R = RbConf;
+  using R = MarchConf<Q>;
   constexpr int NF = U ? 4 : 1, P = R::P, W = R::W, NT = R::NT, KY = R::KY, S = R::S;
-  extern __shared__ __align__(16) float rb_smem[];  // [S slots][NF][H][W]
-  const int lane = threadIdx.x, w = threadIdx.y, t = w * kRbTZ + lane;
-  long long u0 = (long long)blockIdx.x * per_block;
-  const long long uend = min(units, u0 + per_block);
+  constexpr float ga = (float)Tp::gc(1), gd = Q > 7 ? (float)Tp::gc(Q - 1) : 0.f;
+  extern __shared__ __align__(16) float march_smem[];  // [S slots][NF][H][W]
+  let_next();
+  wait_before();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned plane = (unsigned)(g.gy * g.gz);
-  while (u0 < uend) {
-    const int tile = (int)(u0 / g.nx);
-    const int xa = (int)(u0 - (long long)tile * g.nx) + 1;
-    const int xb = (int)min((long long)g.nx, (long long)xa + (uend - u0) - 1);
-    u0 += xb - xa + 1;
+  const F2 a = F2(ga), d = F2(gd), D = F2(Df), half = F2(0.5f), two = F2(2.f);
+  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    const int tile = item % tiles;
+    const int xa = (item / tiles) * len + 1, xb = min(g.nx, xa + len - 1);
     const int z0 = (tile % ntz) * R::TZ, y0 = (tile / ntz) * (R::TY * KY);  // ghosted origin
-    // this thread's tile entries: offset within a plane, or ~0u off the grid
-    unsigned off[R::E];
+    unsigned off[R::E];  // this thread's tile entries within a plane, ~0u off the grid
 #pragma unroll
     for (int k = 0; k < R::E; ++k) {
-      const int e = t + k * NT;
-      const int yy = y0 + e / W, zz = z0 - R::CO + e % W;
-      off[k] = (e < P && yy < g.gy && zz >= 0 && zz < g.gz) ? (unsigned)(yy * g.gz + zz) : ~0u;
+      const int e = (int)threadIdx.x + k * NT;
+      const int yy = y0 + e / W, zz = z0 + e % W;
+      off[k] = (e < P && yy < g.gy && zz < g.gz) ? (unsigned)(yy * g.gz + zz) : ~0u;
     }
-    const int col = R::KZ * lane + 1 + R::CO;  // tile column of the thread's first cell
-    const int z = z0 + R::KZ * lane + 1;
-    auto compute = [&](int x) {
-      const float* sl[3] = {rb_smem + ((x - 1) % S) * NF * P, rb_smem + (x % S) * NF * P,
-                            rb_smem + ((x + 1) % S) * NF * P};
-#pragma unroll
-      for (int rc = 0; rc < KY * R::KZ; ++rc) {
-        const int r = rc / R::KZ, kz = rc % R::KZ;
-        const int ry = w * KY + r + 1;  // tile row of the cell
-        const int y = y0 + ry;
-        // the value of field f at x + e_i; a pair's two middle columns are
-        // one 8-byte load, which the unrolled rows and cells share
-        auto at = [&](int f, int i) -> float {
-          const float* b = sl[1 + Tp::e(i, 0)] + f * P + (ry + Tp::e(i, 1)) * W + col;
-          const int k = kz + Tp::e(i, 2);
-          if (R::KZ == 2 && (k == 0 || k == 1)) {
-            const float2 v = *reinterpret_cast<const float2*>(b);
-            return k == 0 ? v.x : v.y;
-          }
-          return b[k];
-        };
-        const float cnew = fd_cell_links<Q, float, U, CC>([&](int i) { return at(0, i); },
-                                                          [&](int d, int i) { return at(1 + d, i); }, D);
-        if (z + kz <= g.nz && y <= g.ny) cn[(unsigned)x * plane + (unsigned)(y * g.gz + z + kz)] = cnew;
-      }
-    };
-    // planes through registers: plane x + 2 is loaded during plane x and
-    // stored to its slot at the top of the next iteration
-    float r[R::E][NF];
     auto fetch = [&](int xp) {
-      const unsigned pb = (unsigned)xp * plane;
+      if (xp <= xb + 1) {
+        const unsigned pb = (unsigned)xp * plane;
+        float* sp = march_smem + (xp % S) * NF * P + threadIdx.x;
 #pragma unroll
-      for (int k = 0; k < R::E; ++k) {
-        if (off[k] == ~0u) continue;
-        const unsigned a = pb + off[k];
-        r[k][0] = __ldg(c + a);
-        if constexpr (U) {
-          r[k][1] = __ldg(u + a);
-          r[k][2] = __ldg(u + g.L + a);
-          r[k][3] = __ldg(u + 2 * g.L + a);
+        for (int k = 0; k < R::E; ++k) {
+          if (off[k] == ~0u) continue;
+          const unsigned at = pb + off[k];
+          copy_async4(sp + k * NT, c + at);
+          if constexpr (U) {
+            copy_async4(sp + P + k * NT, u + at);
+            copy_async4(sp + 2 * P + k * NT, u + g.L + at);
+            copy_async4(sp + 3 * P + k * NT, u + 2 * g.L + at);
+          }
         }
       }
+      asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto stash = [&](int xp) {
-      float* sp = rb_smem + (xp % S) * NF * P;
-#pragma unroll
-      for (int k = 0; k < R::E; ++k) {
-        if (off[k] == ~0u) continue;
-#pragma unroll
-        for (int f = 0; f < NF; ++f) sp[f * P + t + k * NT] = r[k][f];
-      }
-    };
+    const int z = z0 + 2 * lane + 1, y1 = y0 + w * KY + 1;
+    // outputs of the previous plane, up to that plane's own sums (acc: with
+    // the correction without div and lap, which cl and cd hold), and its centre
+    F2 acc[KY], cl[KY], cd[KY], cc[KY], cu[KY], cv[KY], cw[KY];
+    // the current plane's sums for the next plane's outputs
+    F2 sX[KY], sU[KY], sP[KY], sY[KY], sZ[KY];
     __syncthreads();  // every thread is done with the ring's previous run
     fetch(xa - 1);
-    stash(xa - 1);
     fetch(xa);
-    stash(xa);
-    fetch(xa + 1);
-    for (int x = xa; x <= xb; ++x) {
-      stash(x + 1);     // slot of plane x - 3: nobody reads it any more
-      __syncthreads();  // planes x - 1 .. x + 1 are in
-      if (x < xb) fetch(x + 2);
-      compute(x);
+    for (int x = xa - 1; x <= xb + 1; ++x) {
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();  // plane x is in, plane x - 1 is done with
+      fetch(x + 2);
+      const float* b = march_smem + (x % S) * NF * P + (w * KY) * W + 2 * lane;
+      MarchRow lo = march_row<U, P>(b), mid = march_row<U, P>(b + W);
+#pragma unroll
+      for (int r = 0; r < KY; ++r) {
+        const MarchRow hi = march_row<U, P>(b + (r + 2) * W);
+        // in-plane sums of c
+        const F2 cross = add_(add_(lo.cm, hi.cm), mid.cs), corner = add_(lo.cs, hi.cs);
+        const F2 dy = sub_(hi.cm, lo.cm), dyz = sub_(hi.cs, lo.cs), dzy = add_(lo.cd, hi.cd);
+        // sums that this plane gives the planes before and after it: X with
+        // opposite signs, the others alike
+        auto across = [&](F2 m, F2 m0, F2 m1, F2 s, F2 s0, F2 s1) {
+          F2 t = mul_(a, m);
+          if (Q == 19) t = fma_(d, add_(add_(m0, m1), s), t);
+          if (Q == 15) t = fma_(d, add_(s0, s1), t);
+          return t;
+        };
+        F2 X = mul_(a, mid.cm);
+        if (Q == 19) X = fma_(d, cross, X);
+        if (Q == 15) X = fma_(d, corner, X);
+        F2 Gy = F2(0.f), Gz = F2(0.f), Xu, Xp, Tu = F2(0.f), Tp_ = F2(0.f), v1, v2, q1, q2;
+        if constexpr (U) {
+          Xu = across(mid.um, lo.um, hi.um, mid.us, lo.us, hi.us);
+          Xp = across(mid.pm, lo.pm, hi.pm, mid.ps, lo.ps, hi.ps);
+          v1 = add_(sub_(hi.vm, lo.vm), mid.wd);
+          q1 = add_(sub_(hi.qm, lo.qm), mid.rd);
+          if (Q > 7) {
+            v2 = add_(sub_(hi.vs, lo.vs), add_(lo.wd, hi.wd));
+            q2 = add_(sub_(hi.qs, lo.qs), add_(lo.rd, hi.rd));
+            Gy = mul_(d, Q == 19 ? dy : dyz);
+            Gz = mul_(d, Q == 19 ? mid.cd : dzy);
+            Tu = mul_(d, Q == 19 ? v1 : v2);
+            Tp_ = mul_(d, Q == 19 ? q1 : q2);
+          }
+        }
+        if (x > xa) {
+          // outputs of plane x - 1: this plane's share
+          F2 o = fma_(mul_(two, D), X, acc[r]);
+          if constexpr (U) {
+            const F2 B = add_(Tu, Xu);
+            F2 f = fma_(cc[r], B, add_(Tp_, Xp));
+            f = fma_(cu[r], X, f);
+            if (Q > 7) f = fma_(cw[r], Gz, fma_(cv[r], Gy, f));
+            o = sub_(o, mul_(half, f));
+            if constexpr (CC) {
+              o = div_(o, sub_(F2(1.f), add_(cd[r], B)));
+              const F2 uu = fma_(cw[r], cw[r], fma_(cv[r], cv[r], mul_(cu[r], cu[r])));
+              o = fma_(fma_(two, X, cl[r]), mul_(uu, half), o);
+            }
+          }
+          const int y = y1 + r;
+          if (y <= g.ny) {
+            float* out = cn + (size_t)((unsigned)(x - 1) * plane + (unsigned)(y * g.gz + z));
+            if (z <= g.nz) out[0] = o.lo();
+            if (z < g.nz) out[1] = o.hi();
+          }
+        }
+        if (x >= xa && x <= xb) {
+          // outputs of plane x: the share of plane x - 1 and its own
+          F2 L = fma_(F2((float)Tp::lc(0)), mid.cm, mul_(mul_(two, a), cross));
+          if (Q == 19) L = fma_(mul_(two, d), corner, L);
+          L = fma_(two, sX[r], L);
+          F2 o = fma_(D, L, mid.cm);
+          if constexpr (U) {
+            F2 By = fma_(a, q1, sP[r]), Bu = fma_(a, v1, sU[r]);
+            F2 gy = mul_(a, dy), gz = mul_(a, mid.cd);
+            if (Q == 19) {
+              By = fma_(d, q2, By);
+              Bu = fma_(d, v2, Bu);
+              gy = fma_(d, dyz, gy);
+              gz = fma_(d, dzy, gz);
+            }
+            if (Q > 7) {
+              gy = add_(gy, sY[r]);
+              gz = add_(gz, sZ[r]);
+            }
+            F2 f = fma_(mid.cm, Bu, By);
+            f = fma_(mid.vm, gy, sub_(f, mul_(mid.um, sX[r])));
+            f = fma_(mid.wm, gz, f);
+            o = sub_(o, mul_(half, f));
+            cc[r] = mid.cm;
+            cu[r] = mid.um;
+            cv[r] = mid.vm;
+            cw[r] = mid.wm;
+            if constexpr (CC) {
+              cl[r] = L;
+              cd[r] = Bu;
+            }
+          }
+          acc[r] = o;
+        }
+        sX[r] = X;
+        if constexpr (U) {
+          sU[r] = sub_(Tu, Xu);
+          sP[r] = sub_(Tp_, Xp);
+          sY[r] = Gy;
+          sZ[r] = Gz;
+        }
+        lo = mid;
+        mid = hi;
+      }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
   }
 }
 
@@ -404,6 +450,8 @@ __global__ void k_fd_map_bc(T* __restrict__ c, FdGrid g, const int4* __restrict_
                             const double* __restrict__ wt, const double* __restrict__ nd, int gradient, T value) {
   using Tp = FdTemplate<Q>;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  let_next();
+  wait_before();
   if (t >= n) return;
   const int4 an = cells[t];
   const long long a = ((long long)an.x * g.gy + an.y) * g.gz + an.z;
@@ -489,48 +537,49 @@ cudaError_t fd_launch_one(aslb_fd* f, dim3 grid, dim3 block, const T* c, T* cn, 
     if (e != cudaSuccess) return e;
     raised = true;
   }
-  k_fd_step<Q, T, U, E><<<grid, block, bytes, f->stream>>>(c, cn, u, ef, f->g, T(f->D), U ? f->cc : 0);
-  return cudaGetLastError();
+  return launch_after(k_fd_step<Q, T, U, E>, grid, block, bytes, f->stream, c, cn, u, ef, f->g, T(f->D), U ? f->cc : 0);
 }
 
-// The register-blocked FP32 kernel: one block per resident slot, each with
-// an equal run of the tiles' planes.
+// The marching FP32 kernel on as many blocks as are resident.
 template <int Q, bool U, bool CC>
-cudaError_t fd_launch_rb(aslb_fd* f) {
-  using R = RbConf;
-  constexpr size_t bytes = fd_rb_smem<U>();
-  auto kern = k_fd_step_rb<Q, U, CC>;
+cudaError_t fd_launch_march(aslb_fd* f) {
+  using R = MarchConf<Q>;
+  constexpr size_t bytes = fd_march_smem<Q, U>();
+  auto kern = k_fd_march<Q, U, CC>;
   static int resident = 0;  // blocks per SM
   if (!resident) {
+    int n = 0;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, R::NT, bytes);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, R::NT, bytes);
     if (e != cudaSuccess) return e;
-    if (resident < 1) return cudaErrorInvalidConfiguration;
+    if (n < 1) return cudaErrorInvalidConfiguration;
+    resident = n;
   }
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   const int ntz = (f->g.nz + R::TZ - 1) / R::TZ, nty = (f->g.ny + R::TY * R::KY - 1) / (R::TY * R::KY);
-  const long long units = (long long)ntz * nty * f->g.nx;
-  const long long blocks = std::min<long long>(units, (long long)resident * sms);
-  const long long per_block = (units + blocks - 1) / blocks;
-  kern<<<(unsigned)((units + per_block - 1) / per_block), dim3(kRbTZ, R::TY), bytes, f->stream>>>(
-      (const float*)f->c[f->cur], (float*)f->c[1 - f->cur], (const float*)f->u, f->g, (float)f->D, ntz, units,
-      per_block);
-  return cudaGetLastError();
+  const int tiles = ntz * nty;
+  const long long slots = (long long)resident * sms;
+  // planes per item: one item per block while that keeps them short, else at
+  // most 32 planes (an item reads two planes more than it writes)
+  const long long share = ((long long)tiles * f->g.nx + slots - 1) / slots;
+  const int len = (int)std::min<long long>({share, 32, f->g.nx});
+  const int items = tiles * ((f->g.nx + len - 1) / len);
+  return launch_after(kern, (unsigned)std::min<long long>(items, slots), R::NT, bytes, f->stream,
+                      (const float*)f->c[f->cur], (float*)f->c[1 - f->cur], (const float*)f->u, f->g, (float)f->D, ntz,
+                      tiles, len, items);
 }
 
 template <int Q, class T>
 cudaError_t fd_launch(aslb_fd* f) {
-  // d3q15 / d3q19 in FP32 without the electric term: the register-blocked
-  // kernel; d3q7 (whose update is short and whose step is bound by the
-  // plane fetches, which the smaller tiles below keep more of in flight),
-  // FP64 and the electric term: the 32 x 8 tiles
-  if constexpr (std::is_same<T, float>::value && Q != 7) {
+  // FP32 without the electric term: the marching kernel; FP64 (whose sums
+  // would take twice the registers) and the electric term: the 32 x 8 tiles
+  if constexpr (std::is_same<T, float>::value) {
     if (!f->ef) {
-      if (!f->u) return fd_launch_rb<Q, false, false>(f);
-      return f->cc ? fd_launch_rb<Q, true, true>(f) : fd_launch_rb<Q, true, false>(f);
+      if (!f->u) return fd_launch_march<Q, false, false>(f);
+      return f->cc ? fd_launch_march<Q, true, true>(f) : fd_launch_march<Q, true, false>(f);
     }
   }
   dim3 block(kFdTZ, kFdTY),

@@ -56,6 +56,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// Asynchronous 4-byte copy global -> shared by the calling thread (any 4-byte
+// aligned addresses), part of its open cp.async group.
+__device__ __forceinline__ void copy_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
 // 1-D bulk copy global -> shared, completing on `bar` with `bytes` of
 // transaction count. dst, src and bytes must be multiples of 16 bytes.
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
