@@ -45,11 +45,17 @@ def _stale(target: Path, deps: list[Path]) -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def _file_flags(src: Path) -> list[str]:
+    """The collision writes every multiply-add itself (csrc/collide.cuh), so that all its kernels round alike; contraction
+    would fuse some of its packed products into sums."""
+    return ["--fmad=false"] if src.name.startswith(("step_", "batch_")) else []
+
+
 def _compile(src: Path, extra: list[str], verbose: bool) -> Path:
     out = OBJ / (src.stem + ".o")
     if not _stale(out, [src] + _headers()):
         return out
-    cmd = [nvcc(), *ARCH, *NVCC_FLAGS, *extra, "-c", str(src), "-o", str(out)]
+    cmd = [nvcc(), *ARCH, *NVCC_FLAGS, *_file_flags(src), *extra, "-c", str(src), "-o", str(out)]
     if verbose:
         print(" ".join(cmd), flush=True)
     subprocess.run(cmd, check=True)

@@ -81,9 +81,7 @@ struct aslb_lbgk {
   bool fresh = true;
   std::vector<uint2> mask_host;
   uint2* mask_dev = nullptr;
-  // one word per cell when no cell has both bounce and elide bits (bit 31:
-  // the low bits are elide bits), read by the two-cells-per-thread kernel
-  uint32_t* mask32_dev = nullptr;
+  uint32_t* mask32_dev = nullptr;  // the same in one word per cell, where they fit (link_words)
   // conditions and force objects made on this domain; destroying the domain
   // releases their device memory and detaches them (any destruction order)
   std::vector<aslb_bc*> bcs;
@@ -167,6 +165,11 @@ void prepare_params(aslb_lbgk* h) {
   h->p.cs2 = h->cs2_field;
   h->p.mask = h->fresh ? nullptr : h->mask_dev;
   h->p.mask32 = h->fresh ? nullptr : h->mask32_dev;
+}
+
+// The slot offsets of a domain's grid (StepParams::slot), set once: the
+// opposite-direction searches cost more than a launch.
+void set_slots(aslb_lbgk* h) {
   const GridDesc& g = h->d.g;
   for (int i = 0; i < h->d.q; ++i) {
     const int j = lattice_inv(h->d.q, i);
@@ -470,6 +473,7 @@ int aslb_lbgk_create(int nx, int ny, int nz, int q, int storage, double nu, unsi
     return fail(e == cudaErrorMemoryAllocation ? ASLB_ERR_NOMEM : ASLB_ERR_CUDA, msg);
   }
   h->stream = h->own_stream;
+  set_slots(h);
   h->d.variant = 0;  // direct-load stream-collide by default (measured faster)
   e = cudaMemsetAsync(h->d.F, 0, fbytes, h->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->d.err, 0, sizeof(int), h->stream);
@@ -1433,19 +1437,28 @@ int aslb_bc_fuse(aslb_bc* bc) {
                                 wrapc(h, an.z + lattice_c(q, k, 2), 2));
       add(sa, interior(g, ax, ay, az), sf, k);
     }
-  // the compact form exists when every cell is either a bounce-back reader or
-  // a skipped writer
+  // the one-word form exists when every cell is a bounce-back reader, a
+  // skipped writer, or a skipped writer next to whole fused walls
+  uint32_t wall[6];
+  for (int w = 0; w < 6; ++w) wall[w] = q == 15 ? wall_bits<15>(w) : wall_bits<19>(w);
+  auto one_word = [&](const uint2& w, uint32_t& out) {
+    out = w.y ? (w.y | 0x80000000u) : w.x;
+    if (!w.x || !w.y) return true;
+    uint32_t faces = 0, all = 0;
+    for (int f = 0; f < 6; ++f)
+      if ((w.x & wall[f]) == wall[f]) {
+        faces |= 1u << f;
+        all |= wall[f];
+      }
+    out = kBothLinks | faces << 18 | w.y >> 1;
+    return q < 27 && all == w.x;
+  };
   bool compact = true;
-  for (const uint2& w : m)
-    if (w.x && w.y) {
-      compact = false;
-      break;
-    }
+  std::vector<uint32_t> m32(m.size());
+  for (size_t i = 0; compact && i < m.size(); ++i) compact = one_word(m[i], m32[i]);
   cudaFree(h->mask32_dev);
   h->mask32_dev = nullptr;
   if (compact) {
-    std::vector<uint32_t> m32(m.size());
-    for (size_t i = 0; i < m.size(); ++i) m32[i] = m[i].y ? (m[i].y | 0x80000000u) : m[i].x;
     ASLB_CUDA(cudaMalloc((void**)&h->mask32_dev, ((size_t)g.dstride + 4096) * sizeof(uint32_t)));
     ASLB_CUDA(cudaMemcpy(h->mask32_dev, m32.data(), m32.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
   }
@@ -1698,7 +1711,6 @@ struct aslb_batch {
   long long* dev_starts = nullptr;  // the work split's run tables (BatchWork)
   BatchWork work{};
   bool any_mask = false;
-  int mask_mode = 0;  // 0 no fused links, 1 two-word masks, 2 one-word masks in every masked domain
   std::vector<BatchBc*> dev_pos;  // one table per condition position
   std::vector<int> pos_n;
   std::vector<long long> pos_links;
@@ -1758,7 +1770,6 @@ int batch_tables(aslb_batch* b, aslb_bc* const* bcs, const int* nbc) {
   b->host_doms.assign(n, BatchDom{});
   b->ntiles = 0;
   b->any_mask = false;
-  bool all_m32 = true;
   for (int i = 0; i < n; ++i) {
     aslb_lbgk* h = b->doms[i];
     BatchDom& D = b->host_doms[i];
@@ -1768,7 +1779,7 @@ int batch_tables(aslb_batch* b, aslb_bc* const* bcs, const int* nbc) {
     D.mask = h->fresh ? nullptr : h->mask_dev;
     D.mask32 = h->fresh ? nullptr : h->mask32_dev;
     b->any_mask |= D.mask != nullptr;
-    if (D.mask && !D.mask32) all_m32 = false;
+    b->work.periodic |= g.periodic != 0;
     D.rho = h->d.rho;
     D.u = h->d.u;
     D.om0f = 1.0f / (3.0f * (float)h->p.nu + 0.5f);
@@ -1777,8 +1788,6 @@ int batch_tables(aslb_batch* b, aslb_bc* const* bcs, const int* nbc) {
     D.tile0 = b->ntiles;
     b->ntiles += g.nx;
   }
-  // link-mask form of the launch: 0 none, 1 two words, 2 one word per cell
-  b->mask_mode = b->any_mask ? (all_m32 ? 2 : 1) : 0;
   ASLB_CUDA(cudaMalloc((void**)&b->dev_doms, n * sizeof(BatchDom)));
   ASLB_CUDA(cudaMemcpy(b->dev_doms, b->host_doms.data(), n * sizeof(BatchDom), cudaMemcpyHostToDevice));
   // the work split: contiguous runs of tiles with equal shares of the cells
@@ -1847,7 +1856,7 @@ int batch_step(aslb_batch* b) {
   aslb_lbgk* h0 = b->doms[0];
   prepare_params(h0);
   const int parity = h0->parity;
-  cudaError_t e = launch_batch_step(b->q, b->storage, b->dev_doms, (int)b->doms.size(), b->work, b->mask_mode,
+  cudaError_t e = launch_batch_step(b->q, b->storage, b->dev_doms, (int)b->doms.size(), b->work, b->any_mask,
                                     h0->p, parity, b->shape, b->stream);
   for (size_t j = 0; e == cudaSuccess && j < b->dev_pos.size(); ++j)
     if (b->pos_n[j] > 0)

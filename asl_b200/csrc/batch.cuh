@@ -10,6 +10,7 @@
 // and neighbouring planes of a domain are streamed together.
 // Instantiated per storage in batch_<type>.cu.
 #pragma once
+#include <climits>
 #include "kernels.h"
 #include "stream_collide.cuh"
 #include "bc_links.cuh"
@@ -27,21 +28,31 @@ __host__ __device__ constexpr int batch_shape_blocks(int shape) {
 }
 __host__ __device__ constexpr bool batch_shape_pair(int shape) { return shape >= 3; }
 
-// The fused-link words of a cell: the two-word form, or the one-word form
-// (bit 31 set: the low bits are elide bits, else bounce bits).
-template <bool M32>
+// A domain's fused-link words of a cell, from its one-word masks where it has them.
+template <int Q>
 __device__ __forceinline__ uint2 batch_links(const BatchDom& D, unsigned s) {
-  if (M32) {
-    const uint32_t w = D.mask32[s];
-    return (w >> 31) ? make_uint2(0u, w & 0x7fffffffu) : make_uint2(w, 0u);
+  return D.mask32 ? link_words<Q>(D.mask32[s]) : D.mask[s];
+}
+
+// Neighbour offsets: FLAT when no domain of the batch is periodic (the three
+// displacements per axis are then fixed, and the compiler folds them into one
+// add per population instead of carrying nine selected offsets per cell).
+template <bool FLAT>
+__device__ __forceinline__ void batch_offsets(const GridDesc& g, int x, int y, int z, int (&ox)[3], int (&oy)[3],
+                                              int (&oz)[3]) {
+  if (FLAT) {
+    ox[0] = -(int)g.plane; ox[1] = 0; ox[2] = (int)g.plane;
+    oy[0] = -g.pitch; oy[1] = 0; oy[2] = g.pitch;
+    oz[0] = -1; oz[1] = 0; oz[2] = 1;
+  } else {
+    nb_offsets(g, x, y, z, ox, oy, oz);
   }
-  return D.mask[s];
 }
 
 // Collision and stores of one cell whose store offsets are recomputed after
 // the collision (y and s are made to depend on its result), so the offsets
 // used by the loads die with them instead of living across the collision.
-template <int Q, class S, bool ODD, bool MASKED>
+template <int Q, class S, bool ODD, bool MASKED, bool FLAT>
 __device__ __forceinline__ void batch_finish(S* __restrict__ F, const GridDesc& g, const StepParams& p,
                                              typename MacroT<S>::T* __restrict__ rho_out,
                                              typename MacroT<S>::T* __restrict__ u_out, int x, int y, int z,
@@ -50,7 +61,7 @@ __device__ __forceinline__ void batch_finish(S* __restrict__ F, const GridDesc& 
   cell_collide<Q, S, CL_NONE>(g, p, rho_out, u_out, x, y, z, s, f, om0);
   const int y2 = (int)after((unsigned)y, f[0]);
   int ox[3], oy[3], oz[3];
-  nb_offsets(g, x, y2, z, ox, oy, oz);
+  batch_offsets<FLAT>(g, x, y2, z, ox, oy, oz);
   cell_store<Q, S, ODD, MASKED>(F, p, (unsigned)g.dstride, after(s, f[0]), ox, oy, oz, elide, f);
 }
 
@@ -75,13 +86,15 @@ __device__ __forceinline__ int batch_domain(const BatchDom* __restrict__ doms, i
 // as one sequence of cells 256 at a time, so the next cell's link word is
 // fetched one step ahead across plane boundaries too and the domain's table
 // entry is read once per domain, not once per plane.
-template <int Q, class S, bool ODD, bool FUSED, bool M32, int BLOCKS>
+template <int Q, class S, bool ODD, bool FUSED, bool FLAT, int BLOCKS>
 __global__ void __launch_bounds__(256, BLOCKS)
     k_batch_step(const BatchDom* __restrict__ doms, int ndom, const long long* __restrict__ starts, int K,
                  const StepParams p) {
   using C = typename Store<S>::C;
   using M = typename MacroT<S>::T;
   const int grp = (int)blockIdx.x / K;
+  wait_before();
+  let_next();
   long long tile = starts[grp] + (int)blockIdx.x % K;
   const long long tend = starts[grp + 1];
   int d = -1;
@@ -97,7 +110,7 @@ __global__ void __launch_bounds__(256, BLOCKS)
     const unsigned nz = (unsigned)g.nz, nz_inv = D.nz_inv;
     S* F = (S*)D.F;
     const C om0 = std::is_same<C, double>::value ? C(D.om0d) : C(D.om0f);
-    const bool masked = FUSED && (M32 ? D.mask32 != nullptr : D.mask != nullptr);
+    const bool masked = FUSED && D.mask;
     // storage index of cell l of plane x (y rows of nz cells, z fastest)
     auto cell_index = [&](int x, unsigned l, int& y, int& z) {
       unsigned yq = __umulhi(l, nz_inv);
@@ -116,7 +129,7 @@ __global__ void __launch_bounds__(256, BLOCKS)
     uint2 mnext = make_uint2(0u, 0u);
     if (masked && x <= xb) {
       int y1, z1;
-      mnext = batch_links<M32>(D, cell_index(x, l, y1, z1));
+      mnext = batch_links<Q>(D, cell_index(x, l, y1, z1));
     }
     while (x <= xb) {
       int y, z;
@@ -130,28 +143,30 @@ __global__ void __launch_bounds__(256, BLOCKS)
       }
       if (masked && xn <= xb) {
         int y1, z1;
-        mnext = batch_links<M32>(D, cell_index(xn, ln, y1, z1));
+        mnext = batch_links<Q>(D, cell_index(xn, ln, y1, z1));
       }
       int ox[3], oy[3], oz[3];
-      nb_offsets(g, x, y, z, ox, oy, oz);
+      batch_offsets<FLAT>(g, x, y, z, ox, oy, oz);
       C f[Q];
       cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, s, ox, oy, oz, bounce, f);
-      batch_finish<Q, S, ODD, FUSED>(F, g, p, (M*)D.rho, (M*)D.u, x, y, z, s, elide, f, om0);
+      batch_finish<Q, S, ODD, FUSED, FLAT>(F, g, p, (M*)D.rho, (M*)D.u, x, y, z, s, elide, f, om0);
       x = xn;
       l = ln;
     }
   }
 }
 
-// Two cells per thread: cells l and l + 256 of the plane.
-template <int Q, class S, bool ODD, bool FUSED, bool M32, int BLOCKS>
+// Two cells per thread: cells l and l + 256 of the plane, collided as a pair in
+// packed FP32 (no periodic domain in the batch).
+template <int Q, class S, bool ODD, bool FUSED, int BLOCKS>
 __global__ void __launch_bounds__(256, BLOCKS)
     k_batch_step_pair(const BatchDom* __restrict__ doms, int ndom, const long long* __restrict__ starts, int K,
                       const StepParams p) {
-  using C = typename Store<S>::C;
   using M = typename MacroT<S>::T;
   int d = -1;
   const int grp = (int)blockIdx.x / K;
+  wait_before();
+  let_next();
   const long long tend = starts[grp + 1];
   for (long long tile = starts[grp] + (int)blockIdx.x % K; tile < tend; tile += K) {
     d = batch_domain(doms, ndom, tile, d);
@@ -162,7 +177,7 @@ __global__ void __launch_bounds__(256, BLOCKS)
     const unsigned nz = (unsigned)g.nz, nz_inv = D.nz_inv;
     S* F = (S*)D.F;
     const bool masked = FUSED && D.mask;
-    const C om0 = std::is_same<C, double>::value ? C(D.om0d) : C(D.om0f);
+    const float om0 = D.om0f;
     auto cell_index = [&](unsigned l, int& y, int& z) {
       unsigned yq = __umulhi(l, nz_inv);
       if (yq * nz > l) --yq;
@@ -173,8 +188,8 @@ __global__ void __launch_bounds__(256, BLOCKS)
     uint2 na = make_uint2(0u, 0u), nb = make_uint2(0u, 0u);
     if (masked) {
       int y1, z1;
-      if (threadIdx.x < plane_cells) na = batch_links<M32>(D, cell_index(threadIdx.x, y1, z1));
-      if (threadIdx.x + 256u < plane_cells) nb = batch_links<M32>(D, cell_index(threadIdx.x + 256u, y1, z1));
+      if (threadIdx.x < plane_cells) na = batch_links<Q>(D, cell_index(threadIdx.x, y1, z1));
+      if (threadIdx.x + 256u < plane_cells) nb = batch_links<Q>(D, cell_index(threadIdx.x + 256u, y1, z1));
     }
     for (unsigned l = threadIdx.x; l < plane_cells; l += 512u) {
       const bool has_b = l + 256u < plane_cells;
@@ -184,19 +199,40 @@ __global__ void __launch_bounds__(256, BLOCKS)
       const uint2 ma = na, mb = nb;
       if (masked) {
         int y1, z1;
-        if (l + 512u < plane_cells) na = batch_links<M32>(D, cell_index(l + 512u, y1, z1));
-        if (l + 768u < plane_cells) nb = batch_links<M32>(D, cell_index(l + 768u, y1, z1));
+        if (l + 512u < plane_cells) na = batch_links<Q>(D, cell_index(l + 512u, y1, z1));
+        if (l + 768u < plane_cells) nb = batch_links<Q>(D, cell_index(l + 768u, y1, z1));
       }
-      int ox[3], oya[3], oza[3], oyb[3], ozb[3];
-      nb_offsets(g, x, ya, za, ox, oya, oza);
-      C fa[Q], fb[Q];
-      cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, sa, ox, oya, oza, ma.x, fa);
-      if (has_b) {
-        nb_offsets(g, x, yb, zb, ox, oyb, ozb);
-        cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, sb, ox, oyb, ozb, mb.x, fb);
+      int ox[3], oy[3], oz[3];
+      batch_offsets<true>(g, x, ya, za, ox, oy, oz);
+      float fa[Q], fb[Q];
+      cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, sa, ox, oy, oz, ma.x, fa);
+      if (has_b) cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, sb, ox, oy, oz, mb.x, fb);
+      F2 f[Q], rho, u[3];
+#pragma unroll
+      for (int i = 0; i < Q; ++i) f[i] = F2(fa[i], has_b ? fb[i] : 0.f);
+      collide_cell<Q, F2, CL_NONE, Store<S>::kDev>(f, p, F2(om0), F2(0.f), rho, u);
+      if (p.write_macro) {
+        const long long aa = aidx(g, x, ya, za), ab = aidx(g, x, yb, zb);
+        auto put = [&](M* out, F2 v) {
+          out[aa] = v.lo();
+          if (has_b) out[ab] = v.hi();
+        };
+        if (p.write_rho) put((M*)D.rho, rho);
+        if (p.write_vel) {
+          put((M*)D.u, u[0]);
+          put((M*)D.u + g.L, u[1]);
+          put((M*)D.u + 2 * g.L, u[2]);
+        }
       }
-      batch_finish<Q, S, ODD, FUSED>(F, g, p, (M*)D.rho, (M*)D.u, x, ya, za, sa, ma.y, fa, om0);
-      if (has_b) batch_finish<Q, S, ODD, FUSED>(F, g, p, (M*)D.rho, (M*)D.u, x, yb, zb, sb, mb.y, fb, om0);
+#pragma unroll
+      for (int i = 0; i < Q; ++i) {
+        fa[i] = f[i].lo();
+        fb[i] = f[i].hi();
+      }
+      // store offsets recomputed after the collision (see batch_finish)
+      const unsigned ds2 = after((unsigned)g.dstride, fa[0]);
+      cell_store<Q, S, ODD, FUSED>(F, p, ds2, after(sa, fa[0]), ox, oy, oz, ma.y, fa);
+      if (has_b) cell_store<Q, S, ODD, FUSED>(F, p, ds2, after(sb, fb[0]), ox, oy, oz, mb.y, fb);
     }
   }
 }
@@ -204,68 +240,51 @@ __global__ void __launch_bounds__(256, BLOCKS)
 template <int Q, class S>
 __global__ void __launch_bounds__(256)
     k_batch_links(const BatchBc* __restrict__ bcs, int nbc, long long nlinks, int parity) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nlinks) return;
+  const long long t = min((long long)blockIdx.x * blockDim.x + threadIdx.x, nlinks);
   int lo = 0, hi = nbc - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (bcs[mid].link0 <= t) lo = mid; else hi = mid - 1;
   }
   const BatchBc& B = bcs[lo];
-  link_apply<Q, S>((S*)B.F, B.dstride, B.links, (int)(t - B.link0), B.ls, B.bp, parity);
+  link_apply<Q, S>((S*)B.F, B.dstride, B.links, t < nlinks ? INT_MAX : 0, (int)(t - B.link0), B.ls, B.bp, parity);
 }
 
-template <int Q, class S, int SHAPE, bool M32>
+template <int Q, class S, int SHAPE, bool FLAT>
 cudaError_t batch_step_shape(const BatchDom* doms, int ndom, const BatchWork& w, bool fused, const StepParams& p,
                              int parity_in, cudaStream_t st) {
   constexpr int BLOCKS = batch_shape_blocks(SHAPE);
   const int grid = w.grid[BLOCKS - 2], K = w.group[BLOCKS - 2];
   const long long* starts = w.starts + w.off[BLOCKS - 2];
+  auto go = [&](auto kern) { return launch_after(kern, grid, 256, 0, st, doms, ndom, starts, K, p); };
+  const bool odd = parity_in == 0;
   if constexpr (batch_shape_pair(SHAPE)) {
-    if (parity_in == 0) {
-      if (fused) k_batch_step_pair<Q, S, true, true, M32, BLOCKS><<<grid, 256, 0, st>>>(doms, ndom, starts, K, p);
-      else k_batch_step_pair<Q, S, true, false, false, BLOCKS><<<grid, 256, 0, st>>>(doms, ndom, starts, K, p);
-    } else {
-      if (fused) k_batch_step_pair<Q, S, false, true, M32, BLOCKS><<<grid, 256, 0, st>>>(doms, ndom, starts, K, p);
-      else k_batch_step_pair<Q, S, false, false, false, BLOCKS><<<grid, 256, 0, st>>>(doms, ndom, starts, K, p);
-    }
+    if (odd) return fused ? go(k_batch_step_pair<Q, S, true, true, BLOCKS>) : go(k_batch_step_pair<Q, S, true, false, BLOCKS>);
+    return fused ? go(k_batch_step_pair<Q, S, false, true, BLOCKS>) : go(k_batch_step_pair<Q, S, false, false, BLOCKS>);
   } else {
-    if (parity_in == 0) {
-      if (fused) k_batch_step<Q, S, true, true, M32, BLOCKS><<<grid, 256, 0, st>>>(doms, ndom, starts, K, p);
-      else k_batch_step<Q, S, true, false, false, BLOCKS><<<grid, 256, 0, st>>>(doms, ndom, starts, K, p);
-    } else {
-      if (fused) k_batch_step<Q, S, false, true, M32, BLOCKS><<<grid, 256, 0, st>>>(doms, ndom, starts, K, p);
-      else k_batch_step<Q, S, false, false, false, BLOCKS><<<grid, 256, 0, st>>>(doms, ndom, starts, K, p);
-    }
+    if (odd) return fused ? go(k_batch_step<Q, S, true, true, FLAT, BLOCKS>) : go(k_batch_step<Q, S, true, false, FLAT, BLOCKS>);
+    return fused ? go(k_batch_step<Q, S, false, true, FLAT, BLOCKS>) : go(k_batch_step<Q, S, false, false, FLAT, BLOCKS>);
   }
-  return cudaGetLastError();
 }
 
-// fused: 0 none, 1 two-word link masks, 2 one-word masks in every masked domain
-// Two cells per thread are built for D3Q15 / D3Q19 in 4- and 2-byte storage
-// with one-word link masks (or none); other cases take the one-cell shape
-// with the same residency.
+// Two cells per thread are built for D3Q15 / D3Q19 in 4- and 2-byte storage;
+// other batches take the one-cell shape with the same residency. A batch with
+// a periodic domain has one shape (three blocks, two in FP64).
 template <int Q, class S, int SHAPE>
-cudaError_t batch_step_m(const BatchDom* doms, int ndom, const BatchWork& w, int fused, const StepParams& p,
+cudaError_t batch_step_m(const BatchDom* doms, int ndom, const BatchWork& w, bool fused, const StepParams& p,
                          int parity_in, cudaStream_t st) {
-  if constexpr (batch_shape_pair(SHAPE)) {
-    constexpr int ONE = SHAPE == 3 ? 1 : 2;
-    if constexpr (Q == 27 || sizeof(S) == 8) {
-      return batch_step_m<Q, S, ONE>(doms, ndom, w, fused, p, parity_in, st);
-    } else {
-      if (fused == 1) return batch_step_m<Q, S, ONE>(doms, ndom, w, fused, p, parity_in, st);
-      return batch_step_shape<Q, S, SHAPE, true>(doms, ndom, w, fused != 0, p, parity_in, st);
-    }
-  } else {
-    if (fused == 2) return batch_step_shape<Q, S, SHAPE, true>(doms, ndom, w, true, p, parity_in, st);
-    return batch_step_shape<Q, S, SHAPE, false>(doms, ndom, w, fused != 0, p, parity_in, st);
-  }
+  constexpr int ONE = SHAPE == 3 ? 1 : 2;
+  if constexpr (batch_shape_pair(SHAPE) && (Q == 27 || sizeof(S) == 8))
+    return batch_step_shape<Q, S, ONE, true>(doms, ndom, w, fused, p, parity_in, st);
+  else
+    return batch_step_shape<Q, S, SHAPE, true>(doms, ndom, w, fused, p, parity_in, st);
 }
 
 template <int Q, class S>
 cudaError_t batch_step_impl(const BatchDom* doms, int ndom, const BatchWork& w, int fused, const StepParams& p,
                             int parity_in, int shape, cudaStream_t st) {
   if (w.ntiles <= 0) return cudaSuccess;
+  if (w.periodic) return batch_step_shape<Q, S, sizeof(S) == 8 ? 2 : 1, false>(doms, ndom, w, fused, p, parity_in, st);
   switch (shape) {
     case 0: return batch_step_m<Q, S, 0>(doms, ndom, w, fused, p, parity_in, st);
     case 1: return batch_step_m<Q, S, 1>(doms, ndom, w, fused, p, parity_in, st);
@@ -279,8 +298,7 @@ cudaError_t batch_step_impl(const BatchDom* doms, int ndom, const BatchWork& w, 
 template <int Q, class S>
 cudaError_t batch_links_impl(const BatchBc* bcs, int nbc, long long nlinks, int parity, cudaStream_t st) {
   if (nlinks <= 0) return cudaSuccess;
-  k_batch_links<Q, S><<<(unsigned)((nlinks + 255) / 256), 256, 0, st>>>(bcs, nbc, nlinks, parity);
-  return cudaGetLastError();
+  return launch_after(k_batch_links<Q, S>, (unsigned)((nlinks + 255) / 256), 256, 0, st, bcs, nbc, nlinks, parity);
 }
 
 }  // namespace aslb

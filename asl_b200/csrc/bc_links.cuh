@@ -3,6 +3,7 @@
 #pragma once
 #include <type_traits>
 #include "internal.cuh"
+#include "launch.cuh"
 
 namespace aslb {
 
@@ -28,15 +29,23 @@ struct BcArith {
 // segment table (warp-uniform except at segment ends), the fluid end is
 // anchor + off[k]. A link's IN slot (the population the fluid end streams in
 // next) and OUT slot (that cell's outgoing population in the opposite
-// direction) swap between the AA representations.
+// direction) swap between the AA representations. Threads past the last link
+// (t >= n, n > 0) do nothing.
 template <int Q, class S>
-__device__ __forceinline__ void link_apply(S* __restrict__ F, long long dstride, const int* __restrict__ links, int t,
-                                           const LinkSet& ls, const BcParams& bp, int parity) {
+__device__ __forceinline__ void link_apply(S* __restrict__ F, long long dstride, const int* __restrict__ links, int n,
+                                           int t, const LinkSet& ls, const BcParams& bp, int parity) {
   using C = typename Store<S>::C;
   using A = BcArith<S>;
+  const bool any = t < n;
+  const int tt = any ? t : 0;
+  // direction and anchor are the condition's own data: looked up while the
+  // step before this launch is still finishing
   int k = 1;
-  while (t >= ls.seg[k + 1]) ++k;
-  const int wa = links[t];
+  while (tt >= ls.seg[k + 1]) ++k;
+  const int wa = links[tt];
+  wait_before();
+  let_next();
+  if (!any) return;
   const int wq = wa + ls.off[k];
   const int kb = ls.inv[k];
   S* in;

@@ -26,6 +26,7 @@
 #include <type_traits>
 #include <utility>
 #include "internal.cuh"
+#include "f32x2.cuh"
 #include "mlp.cuh"
 
 namespace aslb {
@@ -43,6 +44,22 @@ __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf
 __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float div_(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ double div_(double a, double b) { return __ddiv_rn(a, b); }
+// a - product: scalar halves, whose explicit rounding is never contracted
+__device__ __forceinline__ float sub_product(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double sub_product(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ F2 sub_product(F2 a, F2 b) { return F2(__fsub_rn(a.lo(), b.lo()), __fsub_rn(a.hi(), b.hi())); }
+__device__ __forceinline__ float sqrt_(float a) { return __fsqrt_rn(a); }
+__device__ __forceinline__ double sqrt_(double a) { return __dsqrt_rn(a); }
+// LBGKTurbulence's limiter: the relaxation rate of a cell whose limiter value
+// is wl (a pair of cells decides per cell).
+template <class C>
+__device__ __forceinline__ C limited_omega(C om0, C wl, C nu) {
+  if (wl > C(1)) return div_(C(1), add_(mul_(C(3), fmin(mul_(nu, wl), C(0.5))), C(0.5)));
+  return om0;
+}
+__device__ __forceinline__ F2 limited_omega(F2 om0, F2 wl, F2 nu) {
+  return F2(limited_omega<float>(om0.lo(), wl.lo(), nu.lo()), limited_omega<float>(om0.hi(), wl.hi(), nu.hi()));
+}
 
 // Compile-time loop: f(std::integral_constant<int, I>) for I = 0 .. N-1.
 template <class F, int... I>
@@ -180,9 +197,9 @@ __device__ __forceinline__ Moments<C> cell_moments(const C (&f)[Q], const StepPa
     // component-sequential, as ACL emits `momentum += (2/w) Omega x momentum`
     const C k = div_(C(2), om0);
     const C O0 = par_Om<C>(p, 0), O1 = par_Om<C>(p, 1), O2 = par_Om<C>(p, 2);
-    m0 = fma_(k, sub_(mul_(O1, m2), mul_(O2, m1)), m0);
-    m1 = fma_(k, sub_(mul_(O2, m0), mul_(O0, m2)), m1);
-    m2 = fma_(k, sub_(mul_(O0, m1), mul_(O1, m0)), m2);
+    m0 = fma_(k, sub_product(mul_(O1, m2), mul_(O2, m1)), m0);
+    m1 = fma_(k, sub_product(mul_(O2, m0), mul_(O0, m2)), m1);
+    m2 = fma_(k, sub_product(mul_(O0, m1), mul_(O1, m0)), m2);
   }
   if (p.has_force) {
     const C hr = DEV ? mul_(mul_(C(0.5), rho), sig) : mul_(C(0.5), rho);
@@ -196,7 +213,7 @@ __device__ __forceinline__ Moments<C> cell_moments(const C (&f)[Q], const StepPa
   const C ium = p.compressible ? (DEV ? mul_(isig, inv_rho) : inv_rho) : isig;
   const C mm = fma_(m2, m2, fma_(m1, m1, mul_(m0, m0)));
   r.a2 = (DEV || p.compressible) ? mul_(C(4.5), ium) : C(4.5);
-  r.a0 = (DEV || p.compressible) ? sub_(V, mul_(mul_(C(1.5), mm), ium)) : sub_(V, mul_(C(1.5), mm));
+  r.a0 = sub_product(V, (DEV || p.compressible) ? mul_(mul_(C(1.5), mm), ium) : mul_(C(1.5), mm));
   r.V = V;
   r.rho = rho;
   r.inv_rho = inv_rho;
@@ -212,22 +229,28 @@ __device__ __forceinline__ Moments<C> cell_moments(const C (&f)[Q], const StepPa
 template <int Q, class C, bool DEV>
 __device__ __forceinline__ void cell_pneq(const C (&f)[Q], const Moments<C>& mo, const StepParams& p, C (&P)[6]) {
   using Lt = Lattice<Q>;
+  using Pr = Pairs<Q>;
+  // Opposite directions have the same products c_a c_b, and the odd parts of
+  // f_eq cancel in their sum, f_eq,i + f_eq,i' = 2 (a0 + a2 (c_i.m)^2), so the
+  // sums run over the pairs: 66 operations for D3Q19 against 170 direction by
+  // direction.
   C P00 = C(0), P11 = C(0), P22 = C(0), P01 = C(0), P12 = C(0), P02 = C(0);
-#pragma unroll
-  for (int i = 0; i < Q; ++i) {
-    const C cm = cdot<Q, C>(i, mo.m0, mo.m1, mo.m2);
-    const C feq = fma_(mo.a2, mul_(cm, cm), fma_(C(3), cm, mo.a0));
-    const C wd = mul_(C(Lt::w(i)), sub_(f[i], feq));
-    if (Lt::c(i, 0) != 0) P00 += wd;
-    if (Lt::c(i, 1) != 0) P11 += wd;
-    if (Lt::c(i, 2) != 0) P22 += wd;
-    if (Lt::c(i, 0) * Lt::c(i, 1) > 0) P01 += wd;
-    if (Lt::c(i, 0) * Lt::c(i, 1) < 0) P01 -= wd;
-    if (Lt::c(i, 1) * Lt::c(i, 2) > 0) P12 += wd;
-    if (Lt::c(i, 1) * Lt::c(i, 2) < 0) P12 -= wd;
-    if (Lt::c(i, 0) * Lt::c(i, 2) > 0) P02 += wd;
-    if (Lt::c(i, 0) * Lt::c(i, 2) < 0) P02 -= wd;
-  }
+  static_for<Q>([&](auto ic) {
+    constexpr int i = decltype(ic)::value;
+    if constexpr (Pr::rep(i)) {
+      const C cm = cdot<Q, C>(i, mo.m0, mo.m1, mo.m2);
+      const C even = fma_(mo.a2, mul_(cm, cm), mo.a0);  // subtracted from each first: those differences round to nothing
+      const C e = add_(sub_(f[i], even), sub_(f[Lt::inv(i)], even));
+      constexpr double w = Lt::w(i);
+      constexpr int xy = Lt::c(i, 0) * Lt::c(i, 1), yz = Lt::c(i, 1) * Lt::c(i, 2), xz = Lt::c(i, 0) * Lt::c(i, 2);
+      if constexpr (Lt::c(i, 0) != 0) P00 = fma_(C(w), e, P00);
+      if constexpr (Lt::c(i, 1) != 0) P11 = fma_(C(w), e, P11);
+      if constexpr (Lt::c(i, 2) != 0) P22 = fma_(C(w), e, P22);
+      if constexpr (xy != 0) P01 = fma_(C(xy * w), e, P01);
+      if constexpr (yz != 0) P12 = fma_(C(yz * w), e, P12);
+      if constexpr (xz != 0) P02 = fma_(C(xz * w), e, P02);
+    }
+  });
   if (DEV) {
     const C isig = C(p.inv_scale);
     P00 = mul_(P00, isig); P11 = mul_(P11, isig); P22 = mul_(P22, isig);
@@ -276,8 +299,7 @@ __device__ __forceinline__ void collide_cell(C (&f)[Q], const StepParams& p, con
       sf = fma_(fa, fa, sf);
     }
     if (DEV) sn = mul_(mul_(sn, isig), isig);
-    const C wl = mul_(C(4), div_(sn, sf));
-    if (wl > C(1)) om = div_(C(1), add_(mul_(C(3), fmin(mul_(par_nu<C>(p), wl), C(0.5))), C(0.5)));
+    om = limited_omega(om0, mul_(C(4), div_(sn, sf)), par_nu<C>(p));
   } else if constexpr (CL == CL_SMAGORINSKY || CL == CL_MLP) {
     // Hou, Sterling, Chen & Doolen (1996): tau = (tau0 + sqrt(tau0^2 + 18 sqrt(2) Cs^2 |Pi_neq| / rho)) / 2,
     // Cs^2 constant (Smagorinsky) or the network's per-cell value (learned closure)
@@ -293,8 +315,8 @@ __device__ __forceinline__ void collide_cell(C (&f)[Q], const StepParams& p, con
     } else {
       cs2 = cs2_cell;
     }
-    const C tau = mul_(C(0.5), add_(tau0, sqrt(fma_(tau0, tau0, mul_(mul_(mul_(C(25.455844122715710), cs2),
-                                                                          sqrt(q2)), inv_rho)))));
+    const C tau = mul_(C(0.5), add_(tau0, sqrt_(fma_(tau0, tau0, mul_(mul_(mul_(C(25.455844122715710), cs2),
+                                                                           sqrt_(q2)), inv_rho)))));
     om = div_(C(1), tau);
   }
 

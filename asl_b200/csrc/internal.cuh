@@ -78,8 +78,8 @@ struct StepParams {
   // slot of a fused link, which the condition would overwrite: the slot keeps
   // its bits (the store is skipped).
   const uint2* mask;
-  // The same links in one word per cell, when no cell has both kinds: bit 31
-  // set = the low bits are elide bits, clear = bounce bits (or null).
+  // The same links in one word per cell, when every cell's fit (link_words),
+  // or null.
   const uint32_t* mask32;
   // Element offsets of the population slots of direction i relative to a
   // cell's storage index s, for cells whose neighbours do not wrap across a
@@ -92,6 +92,32 @@ struct StepParams {
   // the host from the domain's grid, so a population address is one add.
   unsigned slot[4][27];
 };
+
+// The directions that enter a cell from wall w (X0, XE, Y0, YE, Z0, ZE): the
+// bounce bits of a whole wall.
+template <int Q>
+__host__ __device__ constexpr uint32_t wall_bits(int w) {
+  uint32_t m = 0;
+  for (int k = 1; k < Q; ++k)
+    if (Lattice<Q>::c(k, w / 2) == (w % 2 ? -1 : 1)) m |= 1u << k;
+  return m;
+}
+// One-word form of a cell's fused links. Bit 31 clear: the low bits are bounce
+// bits. Bit 31 set, bit 30 clear: elide bits. Both set (D3Q15, D3Q19; a solid
+// cell next to fused walls): elide bits 1 .. 18 in bits 0 .. 17, the walls
+// whose directions bounce in bits 18 .. 23.
+constexpr uint32_t kBothLinks = 0xC0000000u;
+template <int Q>
+__device__ __forceinline__ uint2 link_words(uint32_t w) {
+  if (Q < 27 && w >= kBothLinks) {
+    uint32_t bounce = 0;
+#pragma unroll
+    for (int f = 0; f < 6; ++f)
+      if ((w >> (18 + f)) & 1u) bounce |= wall_bits<Q>(f);
+    return make_uint2(bounce, (w & 0x3ffffu) << 1);
+  }
+  return (w >> 31) ? make_uint2(0u, w & 0x7fffffffu) : make_uint2(w, 0u);
+}
 
 // ---- storage formats -------------------------------------------------------
 template <class S>

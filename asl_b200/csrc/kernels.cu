@@ -80,6 +80,38 @@ __device__ __forceinline__ long long fstar_index(const GridDesc& g, const uint2*
   return (long long)Lt::inv(i) * g.dstride + sq;
 }
 
+// The Q post-collision populations of interior cell (x, y, z): slot F[i][x] or
+// F[inv i][x + c_i], by the parity, the other one for a population that the
+// cell's fused links elide (the cell's own elide bits: the anchor of a link is
+// this cell, so no neighbour's word is needed; with fstar_index, which reads
+// one mask word per direction, the fields of a 384x192x192 porous channel
+// cost 18 more loads per cell). Offsets are p.slot except next to a periodic
+// face.
+template <int Q, class S>
+__device__ __forceinline__ void load_post(const S* __restrict__ F, const GridDesc& g, const StepParams& p, int parity,
+                                          int x, int y, int z, S (&v)[Q]) {
+  using Lt = Lattice<Q>;
+  const unsigned s = (unsigned)sidx(g, x, y, z);
+  unsigned elide = 0;
+  if (p.mask32) elide = link_words<Q>(p.mask32[s]).y;
+  else if (p.mask) elide = p.mask[s].y;
+  if (parity) elide = ~elide;
+  // bit i of elide: take the pushed slot
+  if (wraps(g.periodic & 1, x, g.nx) || wraps(g.periodic & 2, y, g.ny) || wraps(g.periodic & 4, z, g.nz)) {
+    int ox[3], oy[3], oz[3];
+    nb_offsets(g, x, y, z, ox, oy, oz);
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      const unsigned push = (unsigned)Lt::inv(i) * (unsigned)g.dstride +
+                            (unsigned)(ox[1 + Lt::c(i, 0)] + oy[1 + Lt::c(i, 1)] + oz[1 + Lt::c(i, 2)]);
+      v[i] = F[s + (((elide >> i) & 1u) ? push : (unsigned)i * (unsigned)g.dstride)];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < Q; ++i) v[i] = F[s + (((elide >> i) & 1u) ? p.slot[2][i] : p.slot[1][i])];
+  }
+}
+
 // ---------------------------------------------------------------------------
 // initF: f_i = rho (1 + 3 c.u + 4.5 (c.u)^2 - 1.5 u.u) on every ghosted cell
 // (src/num/aslLBGK.cxx:262-280), representation A.
@@ -219,6 +251,8 @@ __global__ void __launch_bounds__(256) k_bc(S* __restrict__ F, const GridDesc g,
   using C = typename Store<S>::C;
   using A = BcArith<S>;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  wait_before();
+  let_next();
   if (t >= n) return;
   const int4 an = anchors[t];
   const unsigned mask = (unsigned)an.w;
@@ -329,8 +363,7 @@ template <int Q, class S>
 static cudaError_t bc_impl(const DomainDev& d, const int4* anchors, int n, const BcParams& bp, int parity,
                            cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_bc<Q, S><<<(n + 255) / 256, 256, 0, st>>>((S*)d.F, d.g, anchors, n, bp, parity);
-  return cudaGetLastError();
+  return launch_after(k_bc<Q, S>, (n + 255) / 256, 256, 0, st, (S*)d.F, d.g, anchors, n, bp, parity);
 }
 
 cudaError_t launch_bc(const DomainDev& d, const int4* anchors, int n, const BcParams& bp, int parity,
@@ -430,16 +463,14 @@ template <int Q, class S>
 __global__ void __launch_bounds__(256) k_bc_links(S* __restrict__ F, const GridDesc g, const int* __restrict__ links,
                                                   int n, const LinkSet ls, const BcParams bp, int parity) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  link_apply<Q, S>(F, g.dstride, links, t, ls, bp, parity);
+  link_apply<Q, S>(F, g.dstride, links, n, t, ls, bp, parity);
 }
 
 template <int Q, class S>
 static cudaError_t bc_links_impl(const DomainDev& d, const int* links, int n, const LinkSet& ls, const BcParams& bp,
                                  int parity, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_bc_links<Q, S><<<(n + 255) / 256, 256, 0, st>>>((S*)d.F, d.g, links, n, ls, bp, parity);
-  return cudaGetLastError();
+  return launch_after(k_bc_links<Q, S>, (n + 255) / 256, 256, 0, st, (S*)d.F, d.g, links, n, ls, bp, parity);
 }
 
 cudaError_t launch_bc_links(const DomainDev& d, const int* links, int n, const LinkSet& ls, const BcParams& bp,
@@ -488,6 +519,8 @@ __global__ void __launch_bounds__(kForceThreads)
   using C = typename Store<S>::C;
   constexpr bool kDev = std::is_same<S, __half>::value;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  wait_before();
+  let_next();
   double v[6] = {0, 0, 0, 0, 0, 0};
   if (t < n) {
     const int4 an = cells[t];
@@ -549,6 +582,8 @@ __global__ void __launch_bounds__(kForceThreads)
 
 __global__ void k_reduce_rows(const double* __restrict__ partials, int nrows, int width, double* __restrict__ out) {
   __shared__ double sh[256];
+  wait_before();
+  let_next();
   for (int j = 0; j < width; ++j) {
     double a = 0.0;
     for (int r = threadIdx.x; r < nrows; r += blockDim.x) a += partials[(size_t)r * width + j];
@@ -564,8 +599,7 @@ __global__ void k_reduce_rows(const double* __restrict__ partials, int nrows, in
 }
 
 cudaError_t launch_reduce_rows(const double* partials, int nblocks, int width, double* out, cudaStream_t st) {
-  k_reduce_rows<<<1, 256, 0, st>>>(partials, nblocks, width, out);
-  return cudaGetLastError();
+  return launch_after(k_reduce_rows, 1, 256, 0, st, partials, nblocks, width, out);
 }
 
 template <int Q, class S>
@@ -573,9 +607,8 @@ static cudaError_t force_impl(const DomainDev& d, const int4* cells, const uint3
                               const double* r0, const double* pos0, double dx, float inv_scale,
                               const uint2* fused, int parity, double* partials, double* out6, cudaStream_t st) {
   const int nb = force_blocks(n);
-  k_force<Q, S><<<nb, kForceThreads, 0, st>>>((const S*)d.F, d.g, cells, mask_in, n, field, r0[0], r0[1], r0[2],
-                                              pos0[0], pos0[1], pos0[2], dx, inv_scale, fused, parity, partials);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_after(k_force<Q, S>, nb, kForceThreads, 0, st, (const S*)d.F, d.g, cells, mask_in, n, field, r0[0],
+                               r0[1], r0[2], pos0[0], pos0[1], pos0[2], dx, inv_scale, fused, parity, partials);
   if (e != cudaSuccess) return e;
   return launch_reduce_rows(partials, nb, 6, out6, st);
 }
@@ -671,9 +704,11 @@ __global__ void __launch_bounds__(kMomentThreads)
     const long long r = c / g.nz;
     const int y = int(r % g.ny) + 1;
     const int x = int(r / g.ny) + 1;
+    S pop[Q];
+    load_post<Q, S>(F, g, p, parity, x, y, z, pop);
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
-      const double fi = double(Store<S>::val(F + fstar_index<Q>(g, p.mask, parity, x, y, z, i), p.inv_scale));
+      const double fi = double(Store<S>::val(&pop[i], p.inv_scale));
       const double wf = Lt::w(i) * fi;
       v[0] += wf;
       v[1] += Lt::c(i, 0) * wf;
@@ -717,11 +752,12 @@ __global__ void __launch_bounds__(kMomentThreads)
     const int y = int(r % g.ny) + 1;
     const int x = int(r / g.ny) + 1;
     double rho = 0, m[3] = {0, 0, 0};
+    S pop[Q];
+    load_post<Q, S>(F, g, p, parity, x, y, z, pop);
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
       // stored populations are f_i / w_i (ASL's layout): rho = sum w f, m = sum w c f
-      const double wf =
-          Lt::w(i) * double(Store<S>::val(F + fstar_index<Q>(g, p.mask, parity, x, y, z, i), p.inv_scale));
+      const double wf = Lt::w(i) * double(Store<S>::val(&pop[i], p.inv_scale));
       rho += wf;
       m[0] += Lt::c(i, 0) * wf;
       m[1] += Lt::c(i, 1) * wf;
@@ -784,13 +820,17 @@ __global__ void __launch_bounds__(256) k_compute_macro(const S* __restrict__ F, 
   using Lt = Lattice<Q>;
   using M = typename MacroT<S>::T;
   const int z = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int y = blockIdx.y + 1;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int x = blockIdx.z + 1;
-  if (z > g.nz) return;
+  wait_before();
+  let_next();
+  if (z > g.nz || y > g.ny) return;
+  S v[Q];
+  load_post<Q, S>(F, g, p, parity, x, y, z, v);
   M rho = M(0), m0 = M(0), m1 = M(0), m2 = M(0);
 #pragma unroll
   for (int i = 0; i < Q; ++i) {
-    const M wf = M(Lt::w(i)) * M(Store<S>::val(F + fstar_index<Q>(g, p.mask, parity, x, y, z, i), p.inv_scale));
+    const M wf = M(Lt::w(i)) * M(Store<S>::val(&v[i], p.inv_scale));
     rho += wf;
     if (Lt::c(i, 0)) m0 += Lt::c(i, 0) > 0 ? wf : -wf;
     if (Lt::c(i, 1)) m1 += Lt::c(i, 1) > 0 ? wf : -wf;
@@ -810,10 +850,10 @@ template <int Q, class S>
 static cudaError_t compute_macro_impl(const DomainDev& d, const StepParams& p, int parity, int comp_rho,
                                       int comp_vel, cudaStream_t st) {
   using M = typename MacroT<S>::T;
-  dim3 block(128), grid((d.g.nz + 127) / 128, d.g.ny, d.g.nx);
-  k_compute_macro<Q, S><<<grid, block, 0, st>>>((const S*)d.F, d.g, p, parity, comp_rho, comp_vel, (M*)d.rho,
-                                                (M*)d.u);
-  return cudaGetLastError();
+  dim3 grid, block;
+  step_launch_shape(d.g, grid, block);
+  return launch_after(k_compute_macro<Q, S>, grid, block, 0, st, (const S*)d.F, d.g, p, parity, comp_rho, comp_vel,
+                      (M*)d.rho, (M*)d.u);
 }
 
 cudaError_t launch_compute_macro(const DomainDev& d, const StepParams& p, int parity, int comp_rho, int comp_vel,

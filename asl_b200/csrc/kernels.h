@@ -103,7 +103,7 @@ struct BatchDom {
   GridDesc g;
   void* F;
   const uint2* mask;  // fused links, or null
-  const uint32_t* mask32;  // the same links in one word per cell (null when a cell has both kinds)
+  const uint32_t* mask32;  // the same links in one word per cell (null when they do not fit)
   void* rho;
   void* u;
   float om0f;
@@ -126,6 +126,7 @@ struct BatchBc {
 // block j of the group every group-th of them from the j-th), one table per
 // residency (2, 3, 4 blocks per SM), back to back in device memory.
 struct BatchWork {
+  bool periodic;  // some domain has a periodic axis
   long long ntiles;
   const long long* starts;  // device
   int grid[3];              // blocks at 2, 3, 4 resident blocks per SM

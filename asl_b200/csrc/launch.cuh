@@ -14,8 +14,10 @@
 
 namespace aslb {
 
-// At the top of a kernel: let the next kernel of the stream launch, then wait
-// for the previous ones.
+// wait_before, then let_next: the next kernel may launch once this one's blocks
+// have all waited. In this order what a kernel reads before its own wait was
+// written before its predecessor began (a list built just before a time loop
+// is visible to the loop's first condition launch, too).
 __device__ __forceinline__ void let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -6,6 +6,7 @@
 #include <type_traits>
 #include "kernels.h"
 #include "collide.cuh"
+#include "launch.cuh"
 
 namespace aslb {
 
@@ -148,6 +149,10 @@ __device__ __forceinline__ unsigned after(unsigned s, float v) {
   asm volatile("" : "+r"(s) : "f"(v));
   return s;
 }
+__device__ __forceinline__ unsigned after(unsigned s, F2 v) {
+  asm volatile("" : "+r"(s) : "l"(v.v));
+  return s;
+}
 __device__ __forceinline__ unsigned after(unsigned s, double v) {
   asm volatile("" : "+r"(s) : "d"(v));
   return s;
@@ -185,17 +190,15 @@ __device__ __forceinline__ bool wraps(int periodic_bit, int v, int n) { return p
 // so the main loop has no branch) and advanced by extra blocks of the same
 // launch, one cell per thread with the wrap-aware offsets (disjoint cells:
 // the AA update of a cell touches only its own slots). The face cells lie on
-// up to eight planes: the two faces of every periodic axis and, with the
-// two-cells-per-thread kernel (which skips both cells of a pair when either
-// wraps), the planes of the z partners of the skipped pairs. A cell on
+// up to six planes, the two faces of every periodic axis. A cell on
 // several planes belongs to the first that holds it. The face blocks come
 // first in the grid (blockIdx.z < fz), so they run alongside the main blocks
 // instead of after them.
 struct FaceWork {
   int n;          // planes
-  int axis[8];
-  int coord[8];
-  int start[9];   // prefix sums of the planes' cell counts
+  int axis[6];
+  int coord[6];
+  int start[7];   // prefix sums of the planes' cell counts
   int fz;         // grid z-slices of face blocks
 };
 
@@ -234,31 +237,23 @@ __device__ __forceinline__ void face_cell(S* __restrict__ F, const GridDesc& g, 
 }
 
 // The face planes of a domain and the grid z-slices their cells need with
-// blocks of `threads` threads on a gx x gy grid face. paired: the main
-// kernel is the two-cells-per-thread kernel, whose pairs are (z, z + 32) for
-// z - 1 mod 64 < 32: with a periodic z it also skips cell 33 (partner of
-// z = 1) and, when nz is the second cell of its pair, cell nz - 32.
+// blocks of `threads` threads on a gx x gy grid face. paired: the main kernel
+// is the two-cells-per-thread kernel, which wraps a periodic z axis itself
+// (its z faces would be single cells of every row, one sector each).
 inline FaceWork face_work(const GridDesc& g, bool paired, int threads, int gx, int gy) {
   FaceWork fw{};
   const int n[3] = {g.nx, g.ny, g.nz};
-  auto add = [&](int a, int c) {
-    for (int j = 0; j < fw.n; ++j)
-      if (fw.axis[j] == a && fw.coord[j] == c) return;
-    fw.axis[fw.n] = a;
-    fw.coord[fw.n] = c;
-    const int cells = (a == 0 ? g.ny * g.nz : (a == 1 ? g.nx * g.nz : g.nx * g.ny));
-    fw.start[fw.n + 1] = fw.start[fw.n] + cells;
-    ++fw.n;
-  };
-  for (int a = 0; a < 3; ++a)
-    if ((g.periodic >> a) & 1) {
-      add(a, 1);
-      add(a, n[a]);
-    }
-  if (paired && (g.periodic & 4)) {
-    if (g.nz >= 33) add(2, 33);
-    if ((g.nz - 1) % 64 >= 32) add(2, g.nz - 32);
-  }
+  for (int a = 0; a < (paired ? 2 : 3); ++a)
+    if ((g.periodic >> a) & 1)
+      for (int side = 0; side < 2; ++side) {
+        const int c = side ? n[a] : 1;
+        if (side && c == 1) continue;
+        const int cells = a == 0 ? g.ny * g.nz : (a == 1 ? g.nx * g.nz : g.nx * g.ny);
+        fw.axis[fw.n] = a;
+        fw.coord[fw.n] = c;
+        fw.start[fw.n + 1] = fw.start[fw.n] + cells;
+        ++fw.n;
+      }
   const long long per_slice = (long long)threads * gx * gy;
   fw.fz = (int)((fw.start[fw.n] + per_slice - 1) / per_slice);
   return fw;
@@ -270,24 +265,26 @@ inline FaceWork face_work(const GridDesc& g, bool paired, int threads, int gx, i
 // F[inv i][x], writes F[i][x]). Element indices are 32-bit (Q * dstride < 2^32).
 // FUSED: the domain has fused no-slip links (p.mask is read); chosen on the
 // host so domains without them run the unmasked code. A block walks
-// kOnePlanes consecutive x planes; with fused links each thread loads the
+// `planes` consecutive x planes; with fused links each thread loads the
 // next plane's link words one iteration ahead (the population addresses
 // depend on them, so they must not cost a second memory round trip).
 constexpr int kOnePlanes = 4;
 template <int Q, class S, int CL, bool ODD, bool FUSED>
 __global__ void __launch_bounds__(256, StepOccupancy<Q, S, CL, FUSED>::blocks)
     k_stream_collide(S* __restrict__ F, const __grid_constant__ GridDesc g, const __grid_constant__ StepParams p,
-                     const __grid_constant__ FaceWork fw, typename MacroT<S>::T* __restrict__ rho_out,
+                     const __grid_constant__ FaceWork fw, int planes, typename MacroT<S>::T* __restrict__ rho_out,
                      typename MacroT<S>::T* __restrict__ u_out) {
   using C = typename Store<S>::C;
+  wait_before();
+  let_next();
   if ((int)blockIdx.z < fw.fz) {
     face_cell<Q, S, CL, ODD, FUSED>(F, g, p, fw, rho_out, u_out);
     return;
   }
   const int z = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  int x0 = (blockIdx.z - fw.fz) * kOnePlanes + 1;
-  int x1 = min(g.nx, x0 + kOnePlanes - 1);
+  int x0 = (blockIdx.z - fw.fz) * planes + 1;
+  int x1 = min(g.nx, x0 + planes - 1);
   if (z > g.nz || y > g.ny) return;
   // cells whose neighbours wrap across a periodic face belong to the face
   // kernel; skipped by the loop's range, the loop body has no branch
@@ -317,42 +314,158 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, CL, FUSED>::blocks)
 
 // Two cells per thread, z and z + 32 of the same row: a warp covers 64
 // consecutive cells, and each thread has the loads of both cells in flight
-// before it collides the first, which doubles the bytes in flight per
-// register-limited warp. Used for the plain (no closure) FP32 and FP16 steps
-// of D3Q15/D3Q19 domains with fused links, at 768 threads (80 registers) per
-// SM (FP16 porous channel: 0.704 ms against 0.786 ms with one cell per
-// thread).
-// M32: the links come from the one-word mask (p.mask32). A block walks
-// kPairPlanes consecutive x planes; each thread loads the fused-link words of
-// the next plane one iteration ahead, so that the population loads, whose
-// addresses those words select, do not wait for a second memory round trip.
+// before it collides them. FP32 and FP16 storage: with fused links, and
+// without them for the closures and for a periodic z axis, which
+// wraps in the lane's own offsets (a row's first and last cell: as face cells
+// they are one sector per population, and cost a fully periodic 160^3 FP32
+// step 0.156 ms against 0.112). The plain step without links on a z axis that
+// does not wrap is faster with one cell per thread (384x192x192 FP32 0.376 ms
+// against 0.390).
+// A block walks `planes` consecutive x planes; each thread loads the
+// fused-link words of the next plane one iteration ahead, so that the
+// population loads, whose addresses those words select, do not wait for a
+// second memory round trip. x and y faces go to the face blocks.
 constexpr int kPairPlanes = 2;
-// Blocks of 128 threads, six per SM (80 registers, the residency of three
-// 256-thread blocks): the smaller blocks measured 0.8 % faster.
 constexpr int kPairThreads = 128;
-template <int Q, class S, bool ODD, bool FUSED, bool M32>
-__global__ void __launch_bounds__(kPairThreads, 768 / kPairThreads)
-    k_stream_collide_pair(S* __restrict__ F, const __grid_constant__ GridDesc g,
-                          const __grid_constant__ StepParams p, const __grid_constant__ FaceWork fw,
-                          typename MacroT<S>::T* __restrict__ rho_out, typename MacroT<S>::T* __restrict__ u_out) {
-  using C = typename Store<S>::C;
+// Resident blocks of 128 threads: six (80 registers) for D3Q15 / D3Q19 with
+// fused links, five (96) without (the compiler hoists the addresses), four
+// (128) for D3Q27; the closures without links take five in the odd step (three
+// bases keep fewer addresses live) and four in the even one, three to four in
+// D3Q27.
+template <int Q, int CL, bool MASKED, bool ODD>
+constexpr int kPairBlocks = Q == 27 ? (CL == CL_NONE || (ODD && !MASKED) ? 4 : 3)
+                                    : (CL == CL_NONE ? (MASKED ? 6 : 5) : (ODD && !MASKED ? 5 : 4));
+// Whether the collision runs on the pair in packed FP32 (f32x2.cuh): where
+// the link selects of D3Q15 / D3Q19 do not dominate, it halves the collision's
+// instructions (160^3 periodic FP32, ms per step packed / scalar: plain 0.112
+// / 0.134, Smagorinsky 0.138 / 0.155, learned closure at 128^3 0.064 / 0.082;
+// D3Q27 with links 0.198 / 0.206; with links FP16 D3Q19 0.362 / 0.355).
+template <int Q, int CL, bool MASKED>
+constexpr bool kPairPack = CL != CL_NONE || !MASKED || Q == 27;
+
+// Offsets of a cell and of the cells below and above it along z: the slots at
+// c_z = 0, at z - 1 and at z + 1, wrapped on a periodic z axis.
+struct ZBase {
+  unsigned at, below, above;
+};
+template <bool PZ>
+__device__ __forceinline__ ZBase z_base(const GridDesc& g, unsigned s, int z) {
+  ZBase r;
+  r.at = r.below = r.above = s;
+  if (PZ && (g.periodic & 4)) {
+    if (z == 1) r.below += (unsigned)g.nz;
+    if (z == g.nz) r.above -= (unsigned)g.nz;
+  }
+  return r;
+}
+__device__ __forceinline__ unsigned z_pick(const ZBase& b, int dz) { return dz == 0 ? b.at : (dz < 0 ? b.below : b.above); }
+
+template <int Q, class S, bool ODD, bool MASKED>
+__device__ __forceinline__ void pair_load(const S* __restrict__ F, const ZBase& b, const StepParams& p, uint32_t bounce,
+                                          float (&f)[Q]) {
+  using Lt = Lattice<Q>;
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    unsigned at;
+    if (MASKED) {
+      // ODD: pull, or the opposite own slot when bounced; EVEN: the reverse
+      const bool bb = (bounce >> i) & 1u;
+      at = b.at + ((ODD != bb) ? p.slot[0][i] : p.slot[3][i]);
+    } else {
+      at = ODD ? z_pick(b, -Lt::c(i, 2)) + p.slot[0][i] : b.at + p.slot[3][i];
+    }
+    f[i] = Store<S>::load_c(F + at);
+  }
+}
+template <int Q, class S, bool ODD, bool MASKED>
+__device__ __forceinline__ void pair_store(S* __restrict__ F, const ZBase& b0, const StepParams& p, uint32_t elide,
+                                           const float (&f)[Q]) {
+  using Lt = Lattice<Q>;
+  ZBase b = b0;
+  b.at = after(b.at, f[0]);
+  if (!MASKED) {
+    b.below = after(b.below, f[0]);
+    b.above = after(b.above, f[0]);
+  } else {
+    b.below = b.above = b.at;
+  }
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    const unsigned at = ODD ? z_pick(b, Lt::c(i, 2)) + p.slot[2][i] : b.at + p.slot[1][i];
+    store_slot<S>(F + at, f[i], MASKED && ((elide >> i) & 1u), p);
+  }
+}
+
+// One pair: cells (x, y, za) and, with has_b, (x, y, za + 32) at storage
+// indices sa and sa + 32, with their (bounce, elide) words.
+template <int Q, class S, int CL, bool ODD, bool MASKED>
+__device__ __forceinline__ void pair_step(S* __restrict__ F, const GridDesc& g, const StepParams& p, int x, int y,
+                                          int za, bool has_b, unsigned sa, uint2 ma, uint2 mb,
+                                          float* __restrict__ rho_out, float* __restrict__ u_out) {
+  const unsigned sb = sa + 32u;
+  const int zb = za + 32;
+  const ZBase ba = z_base<!MASKED>(g, sa, za), bb = z_base<!MASKED>(g, sb, zb);
+  float fa[Q], fb[Q];
+  pair_load<Q, S, ODD, MASKED>(F, ba, p, ma.x, fa);
+  if (has_b) pair_load<Q, S, ODD, MASKED>(F, bb, p, mb.x, fb);
+  if constexpr (!kPairPack<Q, CL, MASKED>) {
+    cell_collide<Q, S, CL>(g, p, rho_out, u_out, x, y, za, sa, fa, p.om0f);
+    pair_store<Q, S, ODD, MASKED>(F, ba, p, ma.y, fa);
+    if (has_b) {
+      cell_collide<Q, S, CL>(g, p, rho_out, u_out, x, y, zb, sb, fb, p.om0f);
+      pair_store<Q, S, ODD, MASKED>(F, bb, p, mb.y, fb);
+    }
+  } else {
+    F2 f[Q], rho, u[3], cs2 = F2(0.f);
+    if (CL == CL_MLP) cs2 = F2(p.cs2[sa], has_b ? p.cs2[sb] : 0.f);
+#pragma unroll
+    for (int i = 0; i < Q; ++i) f[i] = F2(fa[i], has_b ? fb[i] : 0.f);
+    collide_cell<Q, F2, CL, Store<S>::kDev>(f, p, F2(p.om0f), cs2, rho, u);
+    if (p.write_macro) {
+      const long long a = aidx(g, x, y, za);
+      auto put = [&](float* out, F2 v) {
+        out[a] = v.lo();
+        if (has_b) out[a + 32] = v.hi();
+      };
+      if (p.write_rho) put(rho_out, rho);
+      if (p.write_vel) {
+        put(u_out, u[0]);
+        put(u_out + g.L, u[1]);
+        put(u_out + 2 * g.L, u[2]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      fa[i] = f[i].lo();
+      fb[i] = f[i].hi();
+    }
+    pair_store<Q, S, ODD, MASKED>(F, ba, p, ma.y, fa);
+    if (has_b) pair_store<Q, S, ODD, MASKED>(F, bb, p, mb.y, fb);
+  }
+}
+
+// FUSED: 0 no links, 1 the two-word masks, 2 the one-word masks.
+template <int Q, class S, int CL, bool ODD, int FUSED>
+__global__ void __launch_bounds__(kPairThreads, kPairBlocks<Q, CL, FUSED != 0, ODD>)
+    k_step_pair(S* __restrict__ F, const __grid_constant__ GridDesc g, const __grid_constant__ StepParams p,
+                const __grid_constant__ FaceWork fw, int planes, float* __restrict__ rho_out,
+                float* __restrict__ u_out) {
+  wait_before();
+  let_next();
   if ((int)blockIdx.z < fw.fz) {
-    face_cell<Q, S, CL_NONE, ODD, FUSED>(F, g, p, fw, rho_out, u_out);
+    face_cell<Q, S, CL, ODD, FUSED != 0>(F, g, p, fw, rho_out, u_out);
     return;
   }
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int za = blockIdx.x * (2 * blockDim.x) + 64 * w + lane + 1;
-  const int zb = za + 32;
   const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  int x0 = (blockIdx.z - fw.fz) * kPairPlanes + 1;
-  int x1 = min(g.nx, x0 + kPairPlanes - 1);
+  int x0 = (blockIdx.z - fw.fz) * planes + 1;
+  int x1 = min(g.nx, x0 + planes - 1);
   if (za > g.nz || y > g.ny) return;
-  const bool has_b = zb <= g.nz;
-  // A pair with a cell whose neighbours wrap across a periodic face is left to
-  // the face kernel (both cells; face_planes lists the partners). Skipping
-  // by the loop's range keeps the loop body free of branches.
-  if (wraps(g.periodic & 2, y, g.ny) || wraps(g.periodic & 4, za, g.nz) || (has_b && (g.periodic & 4) && zb == g.nz))
-    return;
+  const bool has_b = za + 32 <= g.nz;
+  // cells on a periodic x or y face belong to the face blocks; skipped by the
+  // loop's range, the loop body has no branch
+  if (wraps(g.periodic & 2, y, g.ny)) return;
   if (g.periodic & 1) {
     x0 = max(x0, 2);
     x1 = min(x1, g.nx - 1);
@@ -360,46 +473,129 @@ __global__ void __launch_bounds__(kPairThreads, 768 / kPairThreads)
   }
   const unsigned pl = (unsigned)g.plane;
   const unsigned s0 = (unsigned)sidx(g, x0, y, za);
-  const C om0 = step_omega<C>(p);
-  // the fused-link words of the next plane are loaded one plane ahead, so the
-  // population loads (whose addresses they select) never wait for them
-  uint2 wa = make_uint2(0u, 0u), wb = make_uint2(0u, 0u);
-  if (FUSED && M32) {
-    wa.x = p.mask32[s0];
-    if (has_b) wb.x = p.mask32[s0 + 32u];
-  } else if (FUSED) {
-    wa = p.mask[s0];
-    if (has_b) wb = p.mask[s0 + 32u];
-  }
+  auto words = [&](unsigned s) {  // as stored: split when used
+    uint2 v = make_uint2(0u, 0u);
+    if (FUSED == 1) v = p.mask[s];
+    if (FUSED == 2) v.x = p.mask32[s];
+    return v;
+  };
+  auto split = [](uint2 v) { return FUSED == 2 ? link_words<Q>(v.x) : v; };
+  uint2 wa = words(s0), wb = make_uint2(0u, 0u);
+  if (has_b) wb = words(s0 + 32u);
   for (int x = x0; x <= x1; ++x) {
     const unsigned sa = s0 + (unsigned)(x - x0) * pl;
-    const unsigned sb = sa + 32u;
     uint2 na = make_uint2(0u, 0u), nb = make_uint2(0u, 0u);
     if (FUSED && x < x1) {
-      if (M32) {
-        na.x = p.mask32[sa + pl];
-        if (has_b) nb.x = p.mask32[sb + pl];
-      } else {
-        na = p.mask[sa + pl];
-        if (has_b) nb = p.mask[sb + pl];
-      }
+      na = words(sa + pl);
+      if (has_b) nb = words(sa + pl + 32u);
     }
-    uint2 ma = wa, mb = wb;
-    if (FUSED && M32) {
-      ma = (wa.x >> 31) ? make_uint2(0u, wa.x & 0x7fffffffu) : make_uint2(wa.x, 0u);
-      mb = (wb.x >> 31) ? make_uint2(0u, wb.x & 0x7fffffffu) : make_uint2(wb.x, 0u);
-    }
-    C fa[Q], fb[Q];
-    cell_load_flat<Q, S, ODD, FUSED>(F, sa, p, ma.x, fa);
-    if (has_b) cell_load_flat<Q, S, ODD, FUSED>(F, sb, p, mb.x, fb);
-    cell_collide<Q, S, CL_NONE>(g, p, rho_out, u_out, x, y, za, sa, fa, om0);
-    cell_store_flat<Q, S, ODD, FUSED>(F, p, sa, ma.y, fa);
-    if (has_b) {
-      cell_collide<Q, S, CL_NONE>(g, p, rho_out, u_out, x, y, zb, sb, fb, om0);
-      cell_store_flat<Q, S, ODD, FUSED>(F, p, sb, mb.y, fb);
-    }
+    // D3Q27 (the closures' and its own registers leave room for both bodies):
+    // 64 cells without a link take the body without selects
+    if (FUSED && (Q != 27 || __any_sync(__activemask(), wa.x | wa.y | wb.x | wb.y)))
+      pair_step<Q, S, CL, ODD, true>(F, g, p, x, y, za, has_b, sa, split(wa), split(wb), rho_out, u_out);
+    else
+      pair_step<Q, S, CL, ODD, false>(F, g, p, x, y, za, has_b, sa, make_uint2(0u, 0u), make_uint2(0u, 0u), rho_out,
+                                      u_out);
     wa = na;
     wb = nb;
+  }
+}
+
+// FP16 storage without links, rows aligned: two neighbouring cells per thread,
+// z and z + 1 (z odd), so that a population of the two that is not shifted
+// along z is one 4-byte access: all of them in the even step, nine of nineteen
+// in the odd one. Bound by the number of accesses (with one cell per thread a
+// warp's 64-byte loads and stores are as many as FP32's 128-byte ones):
+// 320x208x256 D3Q19, ms per step, 0.269 against 0.342. With fused links the
+// two cells' selects undo it (0.49 against 0.355 for k_step_pair).
+template <int Q, int CL, bool ODD>
+__global__ void __launch_bounds__(kPairThreads, kPairBlocks<Q, CL, CL == CL_NONE, ODD>)
+    k_step_half2(__half* __restrict__ F, const __grid_constant__ GridDesc g, const __grid_constant__ StepParams p,
+                 const __grid_constant__ FaceWork fw, int planes, float* __restrict__ rho_out,
+                 float* __restrict__ u_out) {
+  using Lt = Lattice<Q>;
+  wait_before();
+  let_next();
+  if ((int)blockIdx.z < fw.fz) {
+    face_cell<Q, __half, CL, ODD, false>(F, g, p, fw, rho_out, u_out);
+    return;
+  }
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int za = blockIdx.x * (2 * blockDim.x) + 64 * w + 2 * lane + 1;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  int x0 = (blockIdx.z - fw.fz) * planes + 1;
+  int x1 = min(g.nx, x0 + planes - 1);
+  if (za > g.nz || y > g.ny) return;
+  const bool has_b = za < g.nz;
+  if (wraps(g.periodic & 2, y, g.ny)) return;
+  if (g.periodic & 1) {
+    x0 = max(x0, 2);
+    x1 = min(x1, g.nx - 1);
+  }
+  for (int x = x0; x <= x1; ++x) {
+    const unsigned s = (unsigned)sidx(g, x, y, za);
+    const ZBase ba = z_base<true>(g, s, za), bb = z_base<true>(g, s + 1u, za + 1);
+    float fa[Q], fb[Q];
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      const unsigned off = ODD ? p.slot[0][i] : p.slot[3][i];
+      if (!ODD || Lt::c(i, 2) == 0) {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(F + (s + off)));
+        fa[i] = v.x;
+        fb[i] = v.y;
+      } else {
+        fa[i] = __half2float(F[z_pick(ba, -Lt::c(i, 2)) + off]);
+        fb[i] = has_b ? __half2float(F[z_pick(bb, -Lt::c(i, 2)) + off]) : 0.f;
+      }
+    }
+    if constexpr (CL == CL_NONE) {
+      cell_collide<Q, __half, CL>(g, p, rho_out, u_out, x, y, za, s, fa, p.om0f);
+      if (has_b) cell_collide<Q, __half, CL>(g, p, rho_out, u_out, x, y, za + 1, s + 1u, fb, p.om0f);
+    } else {
+      F2 f[Q], rho, u[3], cs2 = F2(0.f);
+      if (CL == CL_MLP) cs2 = F2(p.cs2[s], has_b ? p.cs2[s + 1u] : 0.f);
+#pragma unroll
+      for (int i = 0; i < Q; ++i) f[i] = F2(fa[i], fb[i]);
+      collide_cell<Q, F2, CL, true>(f, p, F2(p.om0f), cs2, rho, u);
+      if (p.write_macro) {
+        const long long a = aidx(g, x, y, za);
+        auto put = [&](float* out, F2 v) {
+          out[a] = v.lo();
+          if (has_b) out[a + 1] = v.hi();
+        };
+        if (p.write_rho) put(rho_out, rho);
+        if (p.write_vel) {
+          put(u_out, u[0]);
+          put(u_out + g.L, u[1]);
+          put(u_out + 2 * g.L, u[2]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < Q; ++i) {
+        fa[i] = f[i].lo();
+        fb[i] = f[i].hi();
+      }
+    }
+    ZBase sa = ba, sb = bb;
+    sa.at = after(sa.at, fa[0]);
+    sa.below = after(sa.below, fa[0]);
+    sa.above = after(sa.above, fa[0]);
+    sb.at = sa.at + 1u;
+    sb.below = after(sb.below, fb[0]);
+    sb.above = after(sb.above, fb[0]);
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      const unsigned off = ODD ? p.slot[2][i] : p.slot[1][i];
+      const __half2 h = __floats2half2_rn(fa[i], fb[i]);
+      if (!ODD || Lt::c(i, 2) == 0) {
+        __half* at = F + (sa.at + off);
+        if (has_b) *reinterpret_cast<__half2*>(at) = h;
+        else *at = __low2half(h);
+      } else {
+        F[z_pick(sa, Lt::c(i, 2)) + off] = __low2half(h);
+        if (has_b) F[z_pick(sb, Lt::c(i, 2)) + off] = __high2half(h);
+      }
+    }
   }
 }
 
@@ -411,10 +607,20 @@ inline void step_launch_shape(const GridDesc& g, dim3& grid, dim3& block) {
   grid = dim3((g.nz + tz - 1) / tz, (g.ny + ty - 1) / ty, g.nx);
 }
 
-// The one-cell stream-collide: the same blocks, kOnePlanes x planes each.
-inline void plane_launch_shape(const GridDesc& g, dim3& grid, dim3& block) {
+// x planes that a block walks: up to `most`, fewer where that would leave
+// SMs without a block (a small domain's step is one block's chain of planes).
+inline int planes_per_block(const GridDesc& g, const dim3& grid, int most) {
+  int planes = most;
+  while (planes > 1 && (long long)grid.x * grid.y * ((g.nx + planes - 1) / planes) < 4 * 148) planes /= 2;
+  return planes;
+}
+
+// The one-cell stream-collide: the same blocks, several x planes each.
+inline int plane_launch_shape(const GridDesc& g, dim3& grid, dim3& block) {
   step_launch_shape(g, grid, block);
-  grid.z = (g.nx + kOnePlanes - 1) / kOnePlanes;
+  const int planes = planes_per_block(g, grid, kOnePlanes);
+  grid.z = (g.nx + planes - 1) / planes;
+  return planes;
 }
 
 // Launch of the TMA-staged variant (stream_collide_tma.cuh).
@@ -422,12 +628,15 @@ template <int Q, class S, int CL>
 cudaError_t step_tma(const DomainDev& d, const StepParams& p, int parity_in, cudaStream_t st);
 
 // Two-cells-per-thread shape: 32-thread groups cover 64 cells of a row.
-inline void pair_launch_shape(const GridDesc& g, dim3& grid, dim3& block) {
+inline int pair_launch_shape(const GridDesc& g, dim3& grid, dim3& block) {
   int tz = ((g.nz + 63) / 64) * 32;
   if (tz > kPairThreads) tz = kPairThreads;
   int ty = kPairThreads / tz;
   block = dim3(tz, ty, 1);
-  grid = dim3((g.nz + 2 * tz - 1) / (2 * tz), (g.ny + ty - 1) / ty, (g.nx + kPairPlanes - 1) / kPairPlanes);
+  grid = dim3((g.nz + 2 * tz - 1) / (2 * tz), (g.ny + ty - 1) / ty, g.nx);
+  const int planes = planes_per_block(g, grid, kPairPlanes);
+  grid.z = (g.nx + planes - 1) / planes;
+  return planes;
 }
 
 template <int Q, class S, int CL>
@@ -439,33 +648,36 @@ cudaError_t step_q_s_cl(const DomainDev& d, const StepParams& p, int parity_in, 
   S* F = (S*)d.F;
   M* rho = (M*)d.rho;
   M* u = (M*)d.u;
-  if constexpr (CL == CL_NONE && Q != 27 && !std::is_same<S, double>::value) {
-    if (d.variant == 0 && fused) {
-      pair_launch_shape(d.g, grid, block);
+  if constexpr (std::is_same<S, __half>::value) {
+    // even element offsets put z odd on a 4-byte boundary (packed rows need not)
+    if (d.variant == 0 && !fused && (d.g.zoff + 1) % 2 == 0 && d.g.pitch % 2 == 0) {
+      const int planes = pair_launch_shape(d.g, grid, block);
       const FaceWork fw = face_work(d.g, true, block.x * block.y, grid.x, grid.y);
       grid.z += fw.fz;
-      const bool m32 = p.mask32 != nullptr;
-      if (parity_in == 0) {
-        if (m32) k_stream_collide_pair<Q, S, true, true, true><<<grid, block, 0, st>>>(F, d.g, p, fw, rho, u);
-        else k_stream_collide_pair<Q, S, true, true, false><<<grid, block, 0, st>>>(F, d.g, p, fw, rho, u);
-      } else {
-        if (m32) k_stream_collide_pair<Q, S, false, true, true><<<grid, block, 0, st>>>(F, d.g, p, fw, rho, u);
-        else k_stream_collide_pair<Q, S, false, true, false><<<grid, block, 0, st>>>(F, d.g, p, fw, rho, u);
-      }
-      return cudaGetLastError();
+      return launch_after(parity_in == 0 ? k_step_half2<Q, CL, true> : k_step_half2<Q, CL, false>, grid, block, 0, st, F,
+                          d.g, p, fw, planes, rho, u);
     }
   }
-  plane_launch_shape(d.g, grid, block);
+  if constexpr (!std::is_same<S, double>::value) {
+    // two cells per thread: see k_step_pair
+    const bool pz = d.g.periodic & 4;
+    if (d.variant == 0 && (fused ? !pz : (pz || CL != CL_NONE))) {
+      const int planes = pair_launch_shape(d.g, grid, block);
+      const FaceWork fw = face_work(d.g, true, block.x * block.y, grid.x, grid.y);
+      grid.z += fw.fz;
+      auto go = [&](auto kern) { return launch_after(kern, grid, block, 0, st, F, d.g, p, fw, planes, rho, u); };
+      const bool odd = parity_in == 0;
+      if (!fused) return odd ? go(k_step_pair<Q, S, CL, true, 0>) : go(k_step_pair<Q, S, CL, false, 0>);
+      if (!p.mask32) return odd ? go(k_step_pair<Q, S, CL, true, 1>) : go(k_step_pair<Q, S, CL, false, 1>);
+      return odd ? go(k_step_pair<Q, S, CL, true, 2>) : go(k_step_pair<Q, S, CL, false, 2>);
+    }
+  }
+  const int planes = plane_launch_shape(d.g, grid, block);
   const FaceWork fw = face_work(d.g, false, block.x * block.y, grid.x, grid.y);
   grid.z += fw.fz;
-  if (parity_in == 0) {
-    if (fused) k_stream_collide<Q, S, CL, true, true><<<grid, block, 0, st>>>(F, d.g, p, fw, rho, u);
-    else k_stream_collide<Q, S, CL, true, false><<<grid, block, 0, st>>>(F, d.g, p, fw, rho, u);
-  } else {
-    if (fused) k_stream_collide<Q, S, CL, false, true><<<grid, block, 0, st>>>(F, d.g, p, fw, rho, u);
-    else k_stream_collide<Q, S, CL, false, false><<<grid, block, 0, st>>>(F, d.g, p, fw, rho, u);
-  }
-  return cudaGetLastError();
+  auto go = [&](auto kern) { return launch_after(kern, grid, block, 0, st, F, d.g, p, fw, planes, rho, u); };
+  if (parity_in == 0) return fused ? go(k_stream_collide<Q, S, CL, true, true>) : go(k_stream_collide<Q, S, CL, true, false>);
+  return fused ? go(k_stream_collide<Q, S, CL, false, true>) : go(k_stream_collide<Q, S, CL, false, false>);
 }
 
 template <int Q, class S>

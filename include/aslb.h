@@ -212,8 +212,8 @@ int aslb_lbgk_step_commit(aslb_lbgk* h);
  * bounded wait gave up. */
 int aslb_lbgk_sync(aslb_lbgk* h);
 /* Stream-collide kernel variant: 0 (default) loads directly, two cells per
- * thread for the plain FP32/FP16 D3Q15/D3Q19 step with fused no-slip links
- * (one cell per thread otherwise); 1 stages
+ * thread in FP32 / FP16 where that is faster (fused no-slip links, closures, a
+ * periodic z axis, FP16 without links), one cell per thread otherwise; 1 stages
  * every tile's population rows in shared memory with asynchronous bulk copies
  * (TMA) in a persistent, pipelined kernel; 2 loads directly, one cell per
  * thread. All give identical results. */

@@ -1,0 +1,126 @@
+"""The stream-collide's two-cells-per-thread kernel and the time loop's merged
+conditions, at the sizes where they change form, against the one-cell kernel
+and the separate launches: the same bits (the packed collision rounds each
+cell as the scalar one does, and merging only regroups independent copies)."""
+import numpy as np
+import pytest
+
+from asl_b200 import _lib as L
+from asl_b200 import lbgk as A
+from tests.test_gpu_parity import smooth_field, sphere_map
+
+pytestmark = pytest.mark.gpu
+VT = {15: A.d3q15(), 19: A.d3q19(), 27: A.d3q27()}
+
+
+def populations(make, variants=(0, 2)):
+    out = []
+    for v in variants:
+        lb = make(v)
+        out.append((lb.getF(), lb.getVelocity(), lb.getRho()))
+    return out
+
+
+def assert_same(out):
+    for other in out[1:]:
+        for a, b in zip(out[0], other):
+            assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.parametrize("q", [15, 19, 27])
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("closure", [L.CLOSURE_NONE, L.CLOSURE_ASL_INTENT, L.CLOSURE_SMAGORINSKY])
+@pytest.mark.parametrize("nz", [1, 2, 31, 32, 33, 64, 65, 130])
+def test_pair_kernel_wraps_z_and_packs_bitwise(gpu, q, storage, closure, nz):
+    """Rows around one and two cells per lane, with the z axis periodic."""
+    shape = (5, 3, nz)
+    rho, u = smooth_field(tuple(s + 2 for s in shape), nz + q)
+
+    def make(variant):
+        lb = A.LBGK(A.Block(shape), 0.01, VT[q], storage=storage, periodic=(True, nz % 2 == 0, True),
+                    body_force=(1e-4, -2e-4, 1e-4))
+        lb.setKernel(variant)
+        lb.setClosure(closure)
+        A.LBGKUtilities(lb).initF(rho, u)
+        lb.run(5)
+        return lb
+
+    assert_same(populations(make))
+
+
+@pytest.mark.parametrize("q", [15, 19, 27])
+@pytest.mark.parametrize("storage", ["f32", "f16", "f64"])
+@pytest.mark.parametrize("nz", [5, 32, 40, 97])
+def test_fused_sphere_through_a_wall(gpu, q, storage, nz):
+    """A sphere cut by a fused wall has cells with both kinds of links; the
+    fields computed from the populations follow the links too."""
+    shape = (9, 8, nz)
+    m = sphere_map(tuple(s + 2 for s in shape), (4.0, 0.5, nz / 2.0), 2.7)
+    rho, u = smooth_field(tuple(s + 2 for s in shape), 5)
+
+    def make(variant):
+        lb = A.LBGK(A.Block(shape), 0.02, VT[q], storage=storage, periodic=(True, False, False), body_force=(1e-4, 0, 0))
+        lb.setKernel(variant)
+        A.LBGKUtilities(lb).initF(rho, u)
+        bcs = [A.generateBCNoSlip(lb, [A.Y0, A.YE, A.Z0, A.ZE]), A.generateBCNoSlip(lb, m)]
+        for b in bcs:
+            b.fuse()
+        lb.run(7, bcs)
+        A.LBGKUtilities(lb).computeRhoVelocity()
+        return lb
+
+    out = populations(make)
+    assert_same(out)
+    # the fields against the exported populations
+    f, vel, dens_out = out[0]
+    c, w = A.lattice_vectors(q), A.lattice_weights(q)
+    inner = (slice(1, -1),) * 3
+    dens = np.tensordot(w, f, 1)[inner]
+    mom = np.tensordot((w[:, None] * c).T, f, 1)[(slice(None), *inner)]
+    tol = 1e-13 if storage == "f64" else 4e-6  # 27 FP32 terms of size 1
+    assert np.abs(dens_out[inner] - dens).max() < tol
+    assert np.abs(vel[(slice(None), *inner)] - mom / dens).max() < tol
+    lb = make(0)
+    assert np.allclose(lb.moments(), [dens.sum(), *mom.reshape(3, -1).sum(1)], rtol=1e-9, atol=1e-7 * dens.size)
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16", "f64"])
+@pytest.mark.parametrize("case", ["channel", "two_maps", "sphere_at_wall", "periodic", "fused_last"])
+@pytest.mark.parametrize("steps", [7, 24, 43])
+def test_merged_conditions_equal_separate_ones(gpu, storage, case, steps):
+    """run() of 24 steps or more merges consecutive conditions (and of 32 or more
+    replays eight steps at a time); walls share edge links (the later
+    condition's value stays), and two maps whose links read each other's slots
+    are left separate."""
+    shape = (14, 10, 9)
+    g = tuple(s + 2 for s in shape)
+    rho, u = smooth_field(g, 11, amp=0.02)
+    out = []
+    for merged in (True, False):
+        lb = A.LBGK(A.Block(shape), 0.03, A.d3q19(), storage=storage, periodic=(False, False, case == "periodic"))
+        A.LBGKUtilities(lb).initF(rho, u)
+        walls = [A.Y0, A.YE] + ([] if case == "periodic" else [A.Z0, A.ZE])
+        bcs = [A.generateBCConstantVelocity(lb, (0.03, 0.01, 0.0), [A.X0]), A.generateBCNoSlip(lb, walls),
+               A.generateBCConstantPressure(lb, 1.01, [A.XE])]
+        if case == "two_maps":
+            bcs.append(A.generateBCNoSlip(lb, sphere_map(g, (5.0, 5.0, 4.0), 2.0)))
+            bcs.append(A.generateBCConstantPressure(lb, 1.02, -sphere_map(g, (5.0, 5.0, 4.0), 2.0)))
+        elif case == "sphere_at_wall":
+            bcs.append(A.generateBCNoSlip(lb, sphere_map(g, (6.0, 1.0, 4.0), 2.6)))
+        elif case == "fused_last":
+            bcs.append(A.generateBCNoSlip(lb, sphere_map(g, (6.0, 5.0, 4.0), 2.6)))
+            bcs[-1].fuse()
+        if merged:
+            lb.run(steps, bcs)
+            lb.run(steps, bcs)
+        else:
+            for _ in range(2 * steps):
+                lb.execute()
+                A.executeAll(bcs)
+        out.append((lb.getF(), lb.getVelocity(), lb.getRho()))
+        if merged:  # other condition lists and destroyed conditions
+            lb.run(steps, bcs[:2])
+            del bcs[1]
+            lb.run(steps, bcs)
+            lb.sync()
+    assert_same(out)
