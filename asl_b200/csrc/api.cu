@@ -44,6 +44,13 @@ struct NvtxRange {
   ~NvtxRange() { nvtxRangePop(); }
 };
 
+// Consecutive conditions of a time loop as one launch.
+struct LinkGroup {
+  std::vector<aslb_bc*> bcs;
+  int* links = nullptr;  // device
+  LinkSegs segs{};
+};
+
 struct aslb_lbgk {
   DomainDev d{};
   StepParams p{};
@@ -72,8 +79,13 @@ struct aslb_lbgk {
   cudaGraphExec_t graph = nullptr;
   std::vector<aslb_bc*> graph_bcs;
   int graph_parity = -1;
+  int graph_steps = 0;
   long long graph_version = -1;
   long long version = 0;  // bumped by every parameter change
+  // conditions of the time loop that run as one launch (build_groups), for
+  // the condition list they were built for
+  std::vector<LinkGroup> groups;
+  std::vector<aslb_bc*> groups_key;
   // fused no-slip conditions
   // fresh: populations were (re)initialised and no fused condition has run
   // since, so incoming slots still hold their initial values and the next
@@ -186,10 +198,13 @@ bool mlp_due(const aslb_lbgk* h) {
   return h->closure == CL_MLP && (h->mlp_last < 0 || h->steps - h->mlp_last >= h->mlp_period);
 }
 
-// Steps of one replayed time-loop graph: two (the AA parities), or a whole
-// refresh period of the learned closure (even, so it starts on one parity).
-int graph_cycle(const aslb_lbgk* h) {
-  if (h->closure != CL_MLP) return 2;
+// Steps of a time-loop graph recorded for a run of nsteps: two (the AA
+// parities), or a whole refresh period of the learned closure (even, so it
+// starts on one parity). Long runs of small domains record eight: the kernels
+// of one replay follow each other as dependent launches, replays do not, and
+// that gap (about 2 us) is a tenth of such a step.
+int graph_cycle(const aslb_lbgk* h, int nsteps) {
+  if (h->closure != CL_MLP) return nsteps >= 32 && h->d.g.L < (1 << 21) ? 8 : 2;
   return h->mlp_period % 2 == 0 ? h->mlp_period : 2 * h->mlp_period;
 }
 
@@ -238,6 +253,12 @@ void drop_graph(aslb_lbgk* h) {
   h->graph = nullptr;
   h->graph_bcs.clear();
   h->graph_parity = -1;
+}
+
+void drop_groups(aslb_lbgk* h) {
+  for (LinkGroup& g : h->groups) cudaFree(g.links);
+  h->groups.clear();
+  h->groups_key.clear();
 }
 
 template <class T>
@@ -497,6 +518,7 @@ int aslb_lbgk_destroy(aslb_lbgk* h) {
   if (!h) return ASLB_OK;
   if (h->stream) cudaStreamSynchronize(h->stream);
   drop_graph(h);
+  drop_groups(h);
   for (aslb_batch* b : std::vector<aslb_batch*>(h->batches)) batch_detach(b, h);
   for (aslb_fd* f : h->fds) fd_detached(f);
   h->fds.clear();
@@ -780,6 +802,149 @@ int aslb_lbgk_step_commit(aslb_lbgk* h) {
   return ASLB_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// ---- conditions of a time loop as one launch ---------------------------------
+// A small domain's step is a chain of short launches, one per condition (2.5
+// to 3 us each on a B200 for walls of a few thousand links). Consecutive
+// direction-sorted conditions can run as one when no link of one reads a slot
+// that a link of another writes, in either representation; a link that a later
+// condition writes too is left to that one (ASL's order: the last writer
+// wins). Above kGroupLinks links a launch is no longer what costs. The check
+// and the copies take about 0.2 ms, so runs of a few steps keep the separate
+// launches.
+constexpr long long kGroupLinks = 1 << 20;
+constexpr int kGroupSteps = 24;
+
+struct LinkRange {  // ascending storage indices, all displaced by off
+  const int* p;
+  const int* e;
+  int off;
+};
+LinkRange incoming(const aslb_bc* b, int k) {
+  return {b->host_links.data() + b->ls.seg[k], b->host_links.data() + b->ls.seg[k + 1], 0};
+}
+LinkRange outgoing(const aslb_bc* b, int k) {  // direction inv k at the fluid ends
+  LinkRange r = incoming(b, k);
+  r.off = b->ls.off[k];
+  return r;
+}
+// Calls f(index in a, index in b) for every common index of two ranges until f
+// returns true; true then. Only the part of each range inside the other's is
+// walked (a wall's links lie in one plane of a channel).
+template <class F>
+bool common(const LinkRange& a, const LinkRange& b, F f) {
+  if (a.p == a.e || b.p == b.e) return false;
+  const int lo = std::max(a.p[0] + a.off, b.p[0] + b.off), hi = std::min(a.e[-1] + a.off, b.e[-1] + b.off);
+  if (lo > hi) return false;
+  const int* i = std::lower_bound(a.p, a.e, lo - a.off);
+  const int* j = std::lower_bound(b.p, b.e, lo - b.off);
+  const int* ie = std::upper_bound(i, a.e, hi - a.off);
+  const int* je = std::upper_bound(j, b.e, hi - b.off);
+  while (i != ie && j != je) {
+    const int d = (*i + a.off) - (*j + b.off);
+    if (d == 0 && f(i - a.p, j - b.p)) return true;
+    i += d <= 0;
+    j += d >= 0;
+  }
+  return false;
+}
+bool conflict(const aslb_bc* a, const aslb_bc* b, int q) {
+  auto yes = [](long long, long long) { return true; };
+  for (int k = 1; k < q; ++k) {
+    const int j = a->ls.inv[k];
+    if (common(outgoing(a, k), incoming(b, j), yes) || common(incoming(a, j), outgoing(b, k), yes)) return true;
+  }
+  return false;
+}
+
+int build_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key) {
+  drop_graph(h);  // it may hold the groups' lists
+  drop_groups(h);
+  const int q = h->d.q;
+  auto plain = [&](const aslb_bc* b) { return !b->field() && !b->fused && b->n == 0 && b->nd > 0; };
+  for (size_t i = 0; i < key.size();) {
+    LinkGroup g;
+    long long links = 0;
+    size_t j = i;
+    for (; j < key.size() && plain(key[j]) && links + key[j]->nd <= kGroupLinks; ++j) {
+      bool ok = key[j]->bp.scale == key[i]->bp.scale;
+      for (size_t m = i; ok && m < j; ++m) ok = key[m] != key[j] && !conflict(key[m], key[j], q);
+      if (!ok) break;
+      links += key[j]->nd;
+      g.bcs.push_back(key[j]);
+    }
+    if (g.bcs.size() < 2) {
+      ++i;
+      continue;
+    }
+    // the conditions' lists one after another, without the links that a later
+    // condition writes
+    std::vector<int> dead;
+    int at = 0;
+    bool fits = true;
+    for (size_t m = 0; m < g.bcs.size() && fits; ++m) {
+      const aslb_bc* b = g.bcs[m];
+      const int mode = b->bp.kind == BCK_NOSLIP || b->bp.kind == BCK_MAP_NOSLIP ? kLinkCopy
+                       : b->bp.kind == BCK_VELOCITY                             ? kLinkAdd
+                                                                                : kLinkSet;
+      for (int k = 1; k < q; ++k) {
+        const LinkRange in = incoming(b, k);
+        if (in.p == in.e) continue;
+        if (g.segs.n == kLinkSegs) {
+          fits = false;
+          break;
+        }
+        const int s = g.segs.n++;
+        g.segs.start[s] = at + b->ls.seg[k];
+        g.segs.in[s] = (unsigned)(k * h->d.g.dstride);
+        g.segs.out[s] = (unsigned)(b->ls.inv[k] * h->d.g.dstride + b->ls.off[k]);
+        g.segs.mode[s] = mode;
+        g.segs.val[s] = b->ls.val[k];
+        g.segs.vald[s] = b->ls.vald[k];
+        for (size_t later = m + 1; later < g.bcs.size(); ++later)
+          common(in, incoming(g.bcs[later], k), [&](long long x, long long) {
+            dead.push_back(at + b->ls.seg[k] + (int)x);
+            return false;
+          });
+      }
+      at += b->nd;
+    }
+    if (fits) {
+      g.segs.start[g.segs.n] = at;
+      // the dropped links' indices follow the lists in the same allocation
+      cudaError_t e = cudaMalloc((void**)&g.links, (at + dead.size()) * sizeof(int));
+      size_t to = 0;
+      for (const aslb_bc* b : g.bcs) {
+        if (e == cudaSuccess)
+          e = cudaMemcpyAsync(g.links + to, b->dlinks, (size_t)b->nd * sizeof(int), cudaMemcpyDeviceToDevice, h->stream);
+        to += b->nd;
+      }
+      if (e == cudaSuccess && !dead.empty()) {
+        e = cudaMemcpyAsync(g.links + at, dead.data(), dead.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream);
+        if (e == cudaSuccess) e = launch_drop_links(g.links, g.links + at, (int)dead.size(), h->stream);
+      }
+      h->groups.push_back(g);  // released with the others
+      if (e == cudaErrorMemoryAllocation) {  // no room: separate launches
+        cudaGetLastError();
+        drop_groups(h);
+        break;
+      }
+      if (e != cudaSuccess) {
+        drop_groups(h);
+        return fail(ASLB_ERR_CUDA, std::string("aslb_lbgk_run: ") + cudaGetErrorString(e));
+      }
+    }
+    i = j;
+  }
+  h->groups_key = key;
+  return ASLB_OK;
+}
+}  // namespace
+
+extern "C" {
+
 int aslb_lbgk_run(aslb_lbgk* h, int nsteps, aslb_bc* const* bcs, int nbc, int use_graph) {
   NvtxRange range("aslb_lbgk_run");
   ASLB_CHECK_HANDLE(h);
@@ -791,18 +956,37 @@ int aslb_lbgk_run(aslb_lbgk* h, int nsteps, aslb_bc* const* bcs, int nbc, int us
   for (int b = 1; b < nbc; ++b)
     if (bcs[b - 1]->fused && !bcs[b]->fused && !bcs[b]->field())
       return fail(ASLB_ERR_ARG, "aslb_lbgk_run: fused conditions must come after all separate ones");
+  const std::vector<aslb_bc*> key(bcs, bcs + nbc);
+  if (nsteps >= kGroupSteps && h->groups_key != key) {
+    // not while a caller records this stream: the lists are allocated and copied
+    cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
+    ASLB_CUDA(cudaStreamIsCapturing(h->stream, &recording));
+    if (recording == cudaStreamCaptureStatusNone) {
+      int r = build_groups(h, key);
+      if (r) return r;
+    }
+  }
+  const std::vector<LinkGroup>* groups = h->groups_key == key ? &h->groups : nullptr;
   auto eager = [&](int n) -> int {
     for (int i = 0; i < n; ++i) {
       int r = do_step(h);
       if (r) return r;
+      size_t next = 0;  // group that comes next in the list
       for (int b = 0; b < nbc; ++b) {
+        if (groups && next < groups->size() && (*groups)[next].bcs[0] == bcs[b]) {
+          const LinkGroup& g = (*groups)[next++];
+          cudaError_t e = launch_bc_merged(h->d, g.links, g.segs, bcs[b]->bp, h->parity, h->stream);
+          if (e != cudaSuccess) return fail(ASLB_ERR_CUDA, std::string("boundary launch: ") + cudaGetErrorString(e));
+          b += (int)g.bcs.size() - 1;
+          continue;
+        }
         r = do_bc(bcs[b]);
         if (r) return r;
       }
     }
     return ASLB_OK;
   };
-  const int cycle = graph_cycle(h);
+  int cycle = graph_cycle(h, nsteps);
   if (!use_graph || h->stream == nullptr || nsteps < cycle) return eager(nsteps);
   int done = 0;
   if (h->macro_once || h->fresh) {
@@ -817,9 +1001,9 @@ int aslb_lbgk_run(aslb_lbgk* h, int nsteps, aslb_bc* const* bcs, int nbc, int us
       if (r) return r;
       done += 1;
     }
-  if (nsteps - done < cycle) return eager(nsteps - done);
-  std::vector<aslb_bc*> key(bcs, bcs + nbc);
   const bool valid = h->graph && h->graph_version == h->version && h->graph_bcs == key;
+  if (valid) cycle = h->graph_steps;
+  if (nsteps - done < cycle) return eager(nsteps - done);
   if (valid && h->graph_parity != h->parity && h->closure != CL_MLP && done < nsteps) {
     int r = eager(1);
     if (r) return r;
@@ -850,6 +1034,7 @@ int aslb_lbgk_run(aslb_lbgk* h, int nsteps, aslb_bc* const* bcs, int nbc, int us
     }
     h->graph_bcs = key;
     h->graph_parity = start_parity;
+    h->graph_steps = cycle;
     h->graph_version = h->version;
   }
   const int reps = (nsteps - done) / cycle;
@@ -1469,6 +1654,7 @@ int aslb_bc_fuse(aslb_bc* bc) {
   bc->fused = true;
   h->version++;
   drop_graph(h);
+  drop_groups(h);
   return ASLB_OK;
 }
 
@@ -1486,6 +1672,7 @@ int aslb_bc_destroy(aslb_bc* bc) {
   if (bc->h) {
     cudaStreamSynchronize(bc->h->stream);
     drop_graph(bc->h);
+    drop_groups(bc->h);
     auto& v = bc->h->bcs;
     v.erase(std::remove(v.begin(), v.end(), bc), v.end());
   }

@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(kFdTZ * kFdTY) k_fd_step(const T* __restrict__
   // three planes of the tile (dynamic: FP64 with velocity and electric fields
   // needs 56 KB)
   extern __shared__ __align__(16) unsigned char fd_smem[];
-  let_next();
   wait_before();
+  let_next();
   auto sm = reinterpret_cast<T(*)[NF][P]>(fd_smem);
   const int tz = threadIdx.x, ty = threadIdx.y, t = ty * kFdTZ + tz;
   const int z0 = blockIdx.x * kFdTZ, y0 = blockIdx.y * kFdTY;  // ghosted origin of the tile
@@ -273,8 +273,8 @@ __global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
   constexpr int NF = U ? 4 : 1, P = R::P, W = R::W, NT = R::NT, KY = R::KY, S = R::S;
   constexpr float ga = (float)Tp::gc(1), gd = Q > 7 ? (float)Tp::gc(Q - 1) : 0.f;
   extern __shared__ __align__(16) float march_smem[];  // [S slots][NF][H][W]
-  let_next();
   wait_before();
+  let_next();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned plane = (unsigned)(g.gy * g.gz);
   const F2 a = F2(ga), d = F2(gd), D = F2(Df), half = F2(0.5f), two = F2(2.f);
@@ -450,8 +450,8 @@ __global__ void k_fd_map_bc(T* __restrict__ c, FdGrid g, const int4* __restrict_
                             const double* __restrict__ wt, const double* __restrict__ nd, int gradient, T value) {
   using Tp = FdTemplate<Q>;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  let_next();
   wait_before();
+  let_next();
   if (t >= n) return;
   const int4 an = cells[t];
   const long long a = ((long long)an.x * g.gy + an.y) * g.gz + an.z;

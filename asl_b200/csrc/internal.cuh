@@ -224,4 +224,20 @@ struct LinkSet {
   double vald[27];
 };
 
+// The segments of a merged launch: links [start[i], start[i + 1]) are one
+// condition's links of one direction. A link's anchor a stands for the slots
+// in[i] + a and out[i] + a of representation A (they swap in B); the incoming
+// slot takes the outgoing one (kLinkCopy), that plus a value (kLinkAdd), or a
+// value (kLinkSet).
+enum LinkMode { kLinkCopy = 0, kLinkAdd = 1, kLinkSet = 2 };
+constexpr int kLinkSegs = 96;
+struct LinkSegs {
+  int n;
+  int start[kLinkSegs + 1];
+  unsigned in[kLinkSegs], out[kLinkSegs];
+  int mode[kLinkSegs];
+  float val[kLinkSegs];
+  double vald[kLinkSegs];
+};
+
 }  // namespace aslb

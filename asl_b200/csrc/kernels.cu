@@ -478,6 +478,60 @@ cudaError_t launch_bc_links(const DomainDev& d, const int* links, int n, const L
   ASLB_DISPATCH(d, bc_links_impl, d, links, n, ls, bp, parity, st)
 }
 
+// Several conditions as one launch. Segment and anchor are the conditions' own
+// data, looked up while the step before this launch is still finishing.
+template <class S>
+__global__ void __launch_bounds__(256) k_bc_merged(S* __restrict__ F, const int* __restrict__ links,
+                                                   const __grid_constant__ LinkSegs t,
+                                                   const __grid_constant__ BcParams bp, int parity) {
+  using C = typename Store<S>::C;
+  using A = BcArith<S>;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int lo = 0, hi = t.n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (t.start[mid] <= i) lo = mid; else hi = mid - 1;
+  }
+  const int a = i < t.start[t.n] ? links[i] : -1;
+  const unsigned in_a = t.in[lo] + (unsigned)a, out_a = t.out[lo] + (unsigned)a;
+  const int mode = t.mode[lo];
+  const C v = std::is_same<C, double>::value ? C(t.vald[lo]) : C(t.val[lo]);
+  wait_before();
+  let_next();
+  if (a < 0) return;
+  S* in = F + (parity == 0 ? in_a : out_a);
+  const S* out = F + (parity == 0 ? out_a : in_a);
+  if (mode == kLinkCopy) *in = *out;
+  else if (mode == kLinkAdd) A::put(in, A::get(out, bp) + v, bp);
+  else A::put(in, A::rep(v), bp);
+}
+
+template <class S>
+static cudaError_t bc_merged_impl(const DomainDev& d, const int* links, const LinkSegs& t, const BcParams& bp, int parity,
+                                  cudaStream_t st) {
+  return launch_after(k_bc_merged<S>, (t.start[t.n] + 255) / 256, 256, 0, st, (S*)d.F, links, t, bp, parity);
+}
+
+cudaError_t launch_bc_merged(const DomainDev& d, const int* links, const LinkSegs& t, const BcParams& bp, int parity,
+                             cudaStream_t st) {
+  switch (d.storage) {
+    case ST_F32: return bc_merged_impl<float>(d, links, t, bp, parity, st);
+    case ST_F16: return bc_merged_impl<__half>(d, links, t, bp, parity, st);
+    case ST_F64: return bc_merged_impl<double>(d, links, t, bp, parity, st);
+  }
+  return cudaErrorInvalidValue;
+}
+
+__global__ void k_drop_links(int* __restrict__ links, const int* __restrict__ dead, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) links[dead[i]] = -1;
+}
+
+cudaError_t launch_drop_links(int* links, const int* dead, int n, cudaStream_t st) {
+  k_drop_links<<<(n + 255) / 256, 256, 0, st>>>(links, dead, n);
+  return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // Reductions: warp shuffle, then one row of partial sums per block.
 template <int W>
