@@ -47,7 +47,7 @@ struct NvtxRange {
 // Consecutive conditions of a time loop as one launch.
 struct LinkGroup {
   std::vector<aslb_bc*> bcs;
-  int* links = nullptr;  // device
+  std::vector<std::vector<int>> dropped;  // per condition: links that a later one writes
   LinkSegs segs{};
 };
 
@@ -255,8 +255,12 @@ void drop_graph(aslb_lbgk* h) {
   h->graph_parity = -1;
 }
 
+cudaError_t mark_dropped(aslb_lbgk* h, aslb_bc* bc, const std::vector<int>& at, bool set);
+
+// Forget the merged launches; their conditions (still alive) lose the marks.
 void drop_groups(aslb_lbgk* h) {
-  for (LinkGroup& g : h->groups) cudaFree(g.links);
+  for (LinkGroup& g : h->groups)
+    for (size_t m = 0; m < g.bcs.size(); ++m) mark_dropped(h, g.bcs[m], g.dropped[m], false);
   h->groups.clear();
   h->groups_key.clear();
 }
@@ -516,9 +520,9 @@ void batch_detach(aslb_batch* b, aslb_lbgk* h);
 
 int aslb_lbgk_destroy(aslb_lbgk* h) {
   if (!h) return ASLB_OK;
+  drop_groups(h);
   if (h->stream) cudaStreamSynchronize(h->stream);
   drop_graph(h);
-  drop_groups(h);
   for (aslb_batch* b : std::vector<aslb_batch*>(h->batches)) batch_detach(b, h);
   for (aslb_fd* f : h->fds) fd_detached(f);
   h->fds.clear();
@@ -812,10 +816,11 @@ namespace {
 // that a link of another writes, in either representation; a link that a later
 // condition writes too is left to that one (ASL's order: the last writer
 // wins). Above kGroupLinks links a launch is no longer what costs. The check
-// and the copies take about 0.2 ms, so runs of a few steps keep the separate
-// launches.
+// and the marks take some tens of microseconds once per condition list, and
+// nothing is allocated: the launch reads the conditions' own lists.
 constexpr long long kGroupLinks = 1 << 20;
-constexpr int kGroupSteps = 24;
+constexpr size_t kGroupDropped = 16384;
+constexpr int kGroupSteps = 4;
 
 struct LinkRange {  // ascending storage indices, all displaced by off
   const int* p;
@@ -859,78 +864,66 @@ bool conflict(const aslb_bc* a, const aslb_bc* b, int q) {
   return false;
 }
 
+cudaError_t mark_dropped(aslb_lbgk* h, aslb_bc* bc, const std::vector<int>& at, bool set) {
+  cudaError_t e = cudaSuccess;
+  LinkMarks m;
+  for (size_t i = 0; e == cudaSuccess && i < at.size(); i += m.n) {
+    m.n = (int)std::min<size_t>(at.size() - i, sizeof(m.at) / sizeof(m.at[0]));
+    std::copy(at.begin() + i, at.begin() + i + m.n, m.at);
+    e = launch_mark_links(bc->dlinks, m, set, h->stream);
+  }
+  return e;
+}
+
 int build_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key) {
-  drop_graph(h);  // it may hold the groups' lists
+  drop_graph(h);  // it may hold merged launches
   drop_groups(h);
   const int q = h->d.q;
   auto plain = [&](const aslb_bc* b) { return !b->field() && !b->fused && b->n == 0 && b->nd > 0; };
   for (size_t i = 0; i < key.size();) {
     LinkGroup g;
-    long long links = 0;
-    size_t j = i;
-    for (; j < key.size() && plain(key[j]) && links + key[j]->nd <= kGroupLinks; ++j) {
+    int links = 0;
+    size_t j = i, dropped = 0;
+    for (; j < key.size() && plain(key[j]) && (long long)links + key[j]->nd <= kGroupLinks; ++j) {
       bool ok = key[j]->bp.scale == key[i]->bp.scale;
       for (size_t m = i; ok && m < j; ++m) ok = key[m] != key[j] && !conflict(key[m], key[j], q);
-      if (!ok) break;
-      links += key[j]->nd;
-      g.bcs.push_back(key[j]);
-    }
-    if (g.bcs.size() < 2) {
-      ++i;
-      continue;
-    }
-    // the conditions' lists one after another, without the links that a later
-    // condition writes
-    std::vector<int> dead;
-    int at = 0;
-    bool fits = true;
-    for (size_t m = 0; m < g.bcs.size() && fits; ++m) {
-      const aslb_bc* b = g.bcs[m];
+      int used = 0;
+      for (int k = 1; k < q; ++k) used += key[j]->ls.seg[k + 1] > key[j]->ls.seg[k];
+      if (!ok || g.segs.n + used > kLinkSegs) break;
+      aslb_bc* b = key[j];
       const int mode = b->bp.kind == BCK_NOSLIP || b->bp.kind == BCK_MAP_NOSLIP ? kLinkCopy
                        : b->bp.kind == BCK_VELOCITY                             ? kLinkAdd
                                                                                 : kLinkSet;
       for (int k = 1; k < q; ++k) {
-        const LinkRange in = incoming(b, k);
-        if (in.p == in.e) continue;
-        if (g.segs.n == kLinkSegs) {
-          fits = false;
-          break;
-        }
+        if (b->ls.seg[k + 1] == b->ls.seg[k]) continue;
         const int s = g.segs.n++;
-        g.segs.start[s] = at + b->ls.seg[k];
+        g.segs.links[s] = b->dlinks + b->ls.seg[k];
+        g.segs.start[s] = links + b->ls.seg[k];
         g.segs.in[s] = (unsigned)(k * h->d.g.dstride);
         g.segs.out[s] = (unsigned)(b->ls.inv[k] * h->d.g.dstride + b->ls.off[k]);
         g.segs.mode[s] = mode;
         g.segs.val[s] = b->ls.val[k];
         g.segs.vald[s] = b->ls.vald[k];
-        for (size_t later = m + 1; later < g.bcs.size(); ++later)
-          common(in, incoming(g.bcs[later], k), [&](long long x, long long) {
-            dead.push_back(at + b->ls.seg[k] + (int)x);
+        // links that this condition writes after an earlier one
+        for (size_t m = 0; m < g.bcs.size(); ++m)
+          common(incoming(g.bcs[m], k), incoming(b, k), [&](long long x, long long) {
+            g.dropped[m].push_back(g.bcs[m]->ls.seg[k] + (int)x);
+            ++dropped;
             return false;
           });
       }
-      at += b->nd;
+      links += b->nd;
+      g.bcs.push_back(b);
+      g.dropped.emplace_back();
     }
-    if (fits) {
-      g.segs.start[g.segs.n] = at;
-      // the dropped links' indices follow the lists in the same allocation
-      cudaError_t e = cudaMalloc((void**)&g.links, (at + dead.size()) * sizeof(int));
-      size_t to = 0;
-      for (const aslb_bc* b : g.bcs) {
-        if (e == cudaSuccess)
-          e = cudaMemcpyAsync(g.links + to, b->dlinks, (size_t)b->nd * sizeof(int), cudaMemcpyDeviceToDevice, h->stream);
-        to += b->nd;
-      }
-      if (e == cudaSuccess && !dead.empty()) {
-        e = cudaMemcpyAsync(g.links + at, dead.data(), dead.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream);
-        if (e == cudaSuccess) e = launch_drop_links(g.links, g.links + at, (int)dead.size(), h->stream);
-      }
-      h->groups.push_back(g);  // released with the others
-      if (e == cudaErrorMemoryAllocation) {  // no room: separate launches
-        cudaGetLastError();
-        drop_groups(h);
-        break;
-      }
+    if (g.bcs.size() < 2 || dropped > kGroupDropped) {
+      ++i;
+      continue;
+    }
+    g.segs.start[g.segs.n] = links;
+    h->groups.push_back(g);
+    for (size_t m = 0; m < g.bcs.size(); ++m) {
+      cudaError_t e = mark_dropped(h, g.bcs[m], g.dropped[m], true);
       if (e != cudaSuccess) {
         drop_groups(h);
         return fail(ASLB_ERR_CUDA, std::string("aslb_lbgk_run: ") + cudaGetErrorString(e));
@@ -957,16 +950,17 @@ int aslb_lbgk_run(aslb_lbgk* h, int nsteps, aslb_bc* const* bcs, int nbc, int us
     if (bcs[b - 1]->fused && !bcs[b]->fused && !bcs[b]->field())
       return fail(ASLB_ERR_ARG, "aslb_lbgk_run: fused conditions must come after all separate ones");
   const std::vector<aslb_bc*> key(bcs, bcs + nbc);
-  if (nsteps >= kGroupSteps && h->groups_key != key) {
-    // not while a caller records this stream: the lists are allocated and copied
-    cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
-    ASLB_CUDA(cudaStreamIsCapturing(h->stream, &recording));
-    if (recording == cudaStreamCaptureStatusNone) {
-      int r = build_groups(h, key);
-      if (r) return r;
-    }
+  // While a caller records this stream, conditions keep their own launches: the
+  // marks are not part of a step, and a recording must not depend on marks that
+  // a later run with other conditions takes back.
+  cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
+  if (nbc > 1) ASLB_CUDA(cudaStreamIsCapturing(h->stream, &recording));
+  if (recording == cudaStreamCaptureStatusNone && nsteps >= kGroupSteps && h->groups_key != key) {
+    int r = build_groups(h, key);
+    if (r) return r;
   }
-  const std::vector<LinkGroup>* groups = h->groups_key == key ? &h->groups : nullptr;
+  const std::vector<LinkGroup>* groups =
+      recording == cudaStreamCaptureStatusNone && h->groups_key == key ? &h->groups : nullptr;
   auto eager = [&](int n) -> int {
     for (int i = 0; i < n; ++i) {
       int r = do_step(h);
@@ -975,7 +969,7 @@ int aslb_lbgk_run(aslb_lbgk* h, int nsteps, aslb_bc* const* bcs, int nbc, int us
       for (int b = 0; b < nbc; ++b) {
         if (groups && next < groups->size() && (*groups)[next].bcs[0] == bcs[b]) {
           const LinkGroup& g = (*groups)[next++];
-          cudaError_t e = launch_bc_merged(h->d, g.links, g.segs, bcs[b]->bp, h->parity, h->stream);
+          cudaError_t e = launch_bc_merged(h->d, g.segs, bcs[b]->bp, h->parity, h->stream);
           if (e != cudaSuccess) return fail(ASLB_ERR_CUDA, std::string("boundary launch: ") + cudaGetErrorString(e));
           b += (int)g.bcs.size() - 1;
           continue;
@@ -1670,9 +1664,9 @@ int aslb_bc_execute(aslb_bc* bc) {
 int aslb_bc_destroy(aslb_bc* bc) {
   if (!bc) return ASLB_OK;
   if (bc->h) {
+    drop_groups(bc->h);
     cudaStreamSynchronize(bc->h->stream);
     drop_graph(bc->h);
-    drop_groups(bc->h);
     auto& v = bc->h->bcs;
     v.erase(std::remove(v.begin(), v.end(), bc), v.end());
   }

@@ -42,7 +42,7 @@ __device__ __forceinline__ void link_apply(S* __restrict__ F, long long dstride,
   // step before this launch is still finishing
   int k = 1;
   while (tt >= ls.seg[k + 1]) ++k;
-  const int wa = links[tt];
+  const int wa = links[tt] & ~kLinkDropped;
   wait_before();
   let_next();
   if (!any) return;

@@ -224,20 +224,30 @@ struct LinkSet {
   double vald[27];
 };
 
-// The segments of a merged launch: links [start[i], start[i + 1]) are one
-// condition's links of one direction. A link's anchor a stands for the slots
+// The segments of a merged launch: its links [start[i], start[i + 1]) are one
+// condition's links of one direction, links[i] its own list of anchors. An
+// anchor with kLinkDropped set belongs to a link that a later condition of the
+// launch writes too (a separate launch of the condition ignores the mark). A
+// link's anchor a stands for the slots
 // in[i] + a and out[i] + a of representation A (they swap in B); the incoming
 // slot takes the outgoing one (kLinkCopy), that plus a value (kLinkAdd), or a
 // value (kLinkSet).
 enum LinkMode { kLinkCopy = 0, kLinkAdd = 1, kLinkSet = 2 };
+constexpr int kLinkDropped = (int)0x80000000;
 constexpr int kLinkSegs = 96;
 struct LinkSegs {
+  const int* links[kLinkSegs];
   int n;
   int start[kLinkSegs + 1];
   unsigned in[kLinkSegs], out[kLinkSegs];
   int mode[kLinkSegs];
   float val[kLinkSegs];
   double vald[kLinkSegs];
+};
+// Links to mark or unmark in one launch.
+struct LinkMarks {
+  int n;
+  int at[512];
 };
 
 }  // namespace aslb

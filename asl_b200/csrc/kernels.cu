@@ -481,8 +481,7 @@ cudaError_t launch_bc_links(const DomainDev& d, const int* links, int n, const L
 // Several conditions as one launch. Segment and anchor are the conditions' own
 // data, looked up while the step before this launch is still finishing.
 template <class S>
-__global__ void __launch_bounds__(256) k_bc_merged(S* __restrict__ F, const int* __restrict__ links,
-                                                   const __grid_constant__ LinkSegs t,
+__global__ void __launch_bounds__(256) k_bc_merged(S* __restrict__ F, const __grid_constant__ LinkSegs t,
                                                    const __grid_constant__ BcParams bp, int parity) {
   using C = typename Store<S>::C;
   using A = BcArith<S>;
@@ -492,7 +491,7 @@ __global__ void __launch_bounds__(256) k_bc_merged(S* __restrict__ F, const int*
     const int mid = (lo + hi + 1) >> 1;
     if (t.start[mid] <= i) lo = mid; else hi = mid - 1;
   }
-  const int a = i < t.start[t.n] ? links[i] : -1;
+  const int a = i < t.start[t.n] ? t.links[lo][i - t.start[lo]] : kLinkDropped;
   const unsigned in_a = t.in[lo] + (unsigned)a, out_a = t.out[lo] + (unsigned)a;
   const int mode = t.mode[lo];
   const C v = std::is_same<C, double>::value ? C(t.vald[lo]) : C(t.val[lo]);
@@ -507,28 +506,29 @@ __global__ void __launch_bounds__(256) k_bc_merged(S* __restrict__ F, const int*
 }
 
 template <class S>
-static cudaError_t bc_merged_impl(const DomainDev& d, const int* links, const LinkSegs& t, const BcParams& bp, int parity,
+static cudaError_t bc_merged_impl(const DomainDev& d, const LinkSegs& t, const BcParams& bp, int parity,
                                   cudaStream_t st) {
-  return launch_after(k_bc_merged<S>, (t.start[t.n] + 255) / 256, 256, 0, st, (S*)d.F, links, t, bp, parity);
+  return launch_after(k_bc_merged<S>, (t.start[t.n] + 255) / 256, 256, 0, st, (S*)d.F, t, bp, parity);
 }
 
-cudaError_t launch_bc_merged(const DomainDev& d, const int* links, const LinkSegs& t, const BcParams& bp, int parity,
-                             cudaStream_t st) {
+cudaError_t launch_bc_merged(const DomainDev& d, const LinkSegs& t, const BcParams& bp, int parity, cudaStream_t st) {
   switch (d.storage) {
-    case ST_F32: return bc_merged_impl<float>(d, links, t, bp, parity, st);
-    case ST_F16: return bc_merged_impl<__half>(d, links, t, bp, parity, st);
-    case ST_F64: return bc_merged_impl<double>(d, links, t, bp, parity, st);
+    case ST_F32: return bc_merged_impl<float>(d, t, bp, parity, st);
+    case ST_F16: return bc_merged_impl<__half>(d, t, bp, parity, st);
+    case ST_F64: return bc_merged_impl<double>(d, t, bp, parity, st);
   }
   return cudaErrorInvalidValue;
 }
 
-__global__ void k_drop_links(int* __restrict__ links, const int* __restrict__ dead, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) links[dead[i]] = -1;
+__global__ void k_mark_links(int* __restrict__ links, const __grid_constant__ LinkMarks m, int set) {
+  const int i = threadIdx.x;
+  if (i >= m.n) return;
+  const int a = links[m.at[i]];
+  links[m.at[i]] = set ? (a | kLinkDropped) : (a & ~kLinkDropped);
 }
 
-cudaError_t launch_drop_links(int* links, const int* dead, int n, cudaStream_t st) {
-  k_drop_links<<<(n + 255) / 256, 256, 0, st>>>(links, dead, n);
+cudaError_t launch_mark_links(int* links, const LinkMarks& m, bool set, cudaStream_t st) {
+  k_mark_links<<<1, 512, 0, st>>>(links, m, set ? 1 : 0);
   return cudaGetLastError();
 }
 

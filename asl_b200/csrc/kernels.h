@@ -64,12 +64,10 @@ cudaError_t launch_bc(const DomainDev& d, const int4* anchors, int n, const BcPa
 // condition except the velocity maps.
 cudaError_t launch_bc_links(const DomainDev& d, const int* links, int n, const LinkSet& ls, const BcParams& bp,
                             int parity, cudaStream_t st);
-// Consecutive conditions as one launch (LinkSegs, internal.cuh): links holds the
-// anchors of all segments, -1 where a later condition writes the link.
-cudaError_t launch_bc_merged(const DomainDev& d, const int* links, const LinkSegs& t, const BcParams& bp, int parity,
-                             cudaStream_t st);
-// links[dead[i]] = -1.
-cudaError_t launch_drop_links(int* links, const int* dead, int n, cudaStream_t st);
+// Consecutive conditions as one launch (LinkSegs, internal.cuh).
+cudaError_t launch_bc_merged(const DomainDev& d, const LinkSegs& t, const BcParams& bp, int parity, cudaStream_t st);
+// Set or clear kLinkDropped of links[m.at[i]].
+cudaError_t launch_mark_links(int* links, const LinkMarks& m, bool set, cudaStream_t st);
 // Surface force: per-cell field (ASL layout, optional) and per-block FP64
 // partial sums of (F, (r - r0) x F), then a fixed-order final sum into out6.
 int force_blocks(int n);

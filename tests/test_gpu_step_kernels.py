@@ -86,9 +86,9 @@ def test_fused_sphere_through_a_wall(gpu, q, storage, nz):
 
 @pytest.mark.parametrize("storage", ["f32", "f16", "f64"])
 @pytest.mark.parametrize("case", ["channel", "two_maps", "sphere_at_wall", "periodic", "fused_last"])
-@pytest.mark.parametrize("steps", [7, 24, 43])
+@pytest.mark.parametrize("steps", [3, 4, 21, 43])
 def test_merged_conditions_equal_separate_ones(gpu, storage, case, steps):
-    """run() of 24 steps or more merges consecutive conditions (and of 32 or more
+    """run() of 4 steps or more merges consecutive conditions (and of 32 or more
     replays eight steps at a time); walls share edge links (the later
     condition's value stays), and two maps whose links read each other's slots
     are left separate."""
