@@ -1965,7 +1965,7 @@ int batch_tables(aslb_batch* b, aslb_bc* const* bcs, const int* nbc) {
     D.u = h->d.u;
     D.om0f = 1.0f / (3.0f * (float)h->p.nu + 0.5f);
     D.om0d = 1.0 / (3.0 * h->p.nu + 0.5);
-    D.nz_inv = (unsigned)((0x100000000ULL + (unsigned long long)g.nz - 1) / (unsigned long long)g.nz);
+    D.nz_inv = (unsigned)std::min(0xffffffffULL, (0x100000000ULL + (unsigned long long)g.nz - 1) / (unsigned long long)g.nz);
     D.tile0 = b->ntiles;
     b->ntiles += g.nx;
   }

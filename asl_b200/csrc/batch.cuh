@@ -113,8 +113,8 @@ __global__ void __launch_bounds__(256, BLOCKS)
     const bool masked = FUSED && D.mask;
     // storage index of cell l of plane x (y rows of nz cells, z fastest)
     auto cell_index = [&](int x, unsigned l, int& y, int& z) {
-      unsigned yq = __umulhi(l, nz_inv);
-      if (yq * nz > l) --yq;  // exact quotient for l < 2^32 / nz
+      unsigned yq = __umulhi(l + 1u, nz_inv);
+      if (yq * nz > l) --yq;  // exact quotient for l < 2^32 / nz - 1
       y = (int)yq + 1;
       z = (int)(l - yq * nz) + 1;
       return (unsigned)sidx(g, x, y, z);
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256, BLOCKS)
     const bool masked = FUSED && D.mask;
     const float om0 = D.om0f;
     auto cell_index = [&](unsigned l, int& y, int& z) {
-      unsigned yq = __umulhi(l, nz_inv);
+      unsigned yq = __umulhi(l + 1u, nz_inv);
       if (yq * nz > l) --yq;
       y = (int)yq + 1;
       z = (int)(l - yq * nz) + 1;

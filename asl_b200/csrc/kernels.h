@@ -112,7 +112,7 @@ struct BatchDom {
   void* u;
   float om0f;
   double om0d;
-  unsigned nz_inv;   // ceil(2^32 / nz): y = l / nz by a multiply-high
+  unsigned nz_inv;   // ceil(2^32 / nz), 2^32 - 1 for nz 1: y = l / nz by a multiply-high of l + 1
   long long tile0;   // first tile (x plane) of this domain in the batch
 };
 // One entry per (domain, condition) of a batched link launch (ordered by link0).

@@ -110,17 +110,52 @@ def test_merged_conditions_equal_separate_ones(gpu, storage, case, steps):
         elif case == "fused_last":
             bcs.append(A.generateBCNoSlip(lb, sphere_map(g, (6.0, 5.0, 4.0), 2.6)))
             bcs[-1].fuse()
-        if merged:
-            lb.run(steps, bcs)
-            lb.run(steps, bcs)
-        else:
-            for _ in range(2 * steps):
-                lb.execute()
-                A.executeAll(bcs)
+        # the same list twice, then others (merged again or dropped), then back
+        for which in (bcs, bcs, bcs[:2], [bcs[0], *bcs[2:]], bcs):
+            if merged:
+                lb.run(steps, which)
+            else:
+                for _ in range(steps):
+                    lb.execute()
+                    A.executeAll(which)
         out.append((lb.getF(), lb.getVelocity(), lb.getRho()))
-        if merged:  # other condition lists and destroyed conditions
-            lb.run(steps, bcs[:2])
-            del bcs[1]
+        if merged:  # a destroyed condition
+            del bcs[1], which
             lb.run(steps, bcs)
             lb.sync()
     assert_same(out)
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("q", [15, 19])
+@pytest.mark.parametrize("shape", [3, 4])
+def test_batch_pairs_across_planes(gpu, q, storage, shape):
+    """Two cells per thread in planes below, at and above a block's cells, so
+    that a pair spans two planes or lacks its second cell; fields included."""
+    sizes = [(3, 1, 1), (7, 5, 9), (5, 6, 1), (4, 16, 20), (9, 17, 19), (2, 32, 20), (1, 40, 33)]
+
+    def domains():
+        out = []
+        for i, size in enumerate(sizes):
+            g = tuple(s + 2 for s in size)
+            lb = A.LBGK(A.Block(size), 0.01 + 0.01 * i, VT[q], storage=storage, body_force=(1e-4, 0, 1e-4), packed_rows=True)
+            A.LBGKUtilities(lb).initF(*smooth_field(g, i, amp=0.02))
+            bcs = [A.generateBCNoSlip(lb, [A.X0, A.XE, A.Y0, A.YE, A.Z0, A.ZE])]
+            if size[0] == 9:
+                bcs.append(A.generateBCNoSlip(lb, sphere_map(g, (5.0, 8.0, 9.0), 3.4)))
+            for b in bcs:
+                b.fuse()
+            out.append((lb, bcs))
+        return out
+
+    alone, together = domains(), domains()
+    for lb, bcs in alone:
+        lb.run(5, bcs)
+        lb.sync()
+    batch = A.Batch([lb for lb, _ in together])
+    batch.setShape(shape)
+    batch.run(5, [bcs for _, bcs in together])
+    batch.sync()
+    for (a, _), (b, _) in zip(alone, together):
+        inner = (..., slice(1, -1), slice(1, -1), slice(1, -1))
+        assert_same([(x.getF(), x.getVelocity()[inner], x.getRho()[inner]) for x in (a, b)])
