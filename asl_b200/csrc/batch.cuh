@@ -19,14 +19,15 @@ namespace aslb {
 
 // Launch shapes of the persistent batched step: one cell per thread at 4, 3
 // or 2 resident blocks of 256 threads per SM (64 / 80 / 128 registers), or
-// two cells per thread (cells l and l + 256 of a plane, both cells' loads in
-// flight before the first collision) at 3 or 2 blocks. aslb_batch_run times
+// two cells per thread (both cells' loads in flight before the collision) at 3
+// blocks of 256 or 2 of 320 threads (80 / 96 registers). aslb_batch_run times
 // them on the batch and keeps the fastest.
 constexpr int kBatchShapes = 5;
 __host__ __device__ constexpr int batch_shape_blocks(int shape) {
   return shape == 0 ? 4 : (shape == 1 || shape == 3 ? 3 : 2);
 }
 __host__ __device__ constexpr bool batch_shape_pair(int shape) { return shape >= 3; }
+__host__ __device__ constexpr int batch_shape_threads(int shape) { return shape == 4 ? 320 : 256; }
 
 // A domain's fused-link words of a cell, from its one-word masks where it has them.
 template <int Q>
@@ -156,10 +157,13 @@ __global__ void __launch_bounds__(256, BLOCKS)
   }
 }
 
-// Two cells per thread: cells l and l + 256 of the plane, collided as a pair in
-// packed FP32 (no periodic domain in the batch).
-template <int Q, class S, bool ODD, bool FUSED, int BLOCKS>
-__global__ void __launch_bounds__(256, BLOCKS)
+// Two cells per thread, NT cells apart in the block's sequence of cells,
+// collided as a pair in packed FP32 (no periodic domain in the batch). The
+// pair too is walked across plane boundaries: the planes of such batches hold
+// two to eight times NT cells, and stopping at each plane's end left a third
+// of the threads without a second cell.
+template <int Q, class S, bool ODD, bool FUSED, int BLOCKS, int NT>
+__global__ void __launch_bounds__(NT, BLOCKS)
     k_batch_step_pair(const BatchDom* __restrict__ doms, int ndom, const long long* __restrict__ starts, int K,
                       const StepParams p) {
   using M = typename MacroT<S>::T;
@@ -167,43 +171,64 @@ __global__ void __launch_bounds__(256, BLOCKS)
   const int grp = (int)blockIdx.x / K;
   wait_before();
   let_next();
+  long long tile = starts[grp] + (int)blockIdx.x % K;
   const long long tend = starts[grp + 1];
-  for (long long tile = starts[grp] + (int)blockIdx.x % K; tile < tend; tile += K) {
+  while (tile < tend) {
     d = batch_domain(doms, ndom, tile, d);
     const BatchDom& D = doms[d];
     const GridDesc g = D.g;
-    const int x = (int)(tile - D.tile0) + 1;
+    // this block's planes of the domain in the run, as in k_batch_step
+    const int x0 = (int)(tile - D.tile0) + 1;
+    const int x1 = (int)(min(tend, D.tile0 + g.nx) - D.tile0);
+    tile += (long long)K * ((x1 - x0) / K + 1);
     const unsigned plane_cells = (unsigned)(g.ny * g.nz);
     const unsigned nz = (unsigned)g.nz, nz_inv = D.nz_inv;
     S* F = (S*)D.F;
     const bool masked = FUSED && D.mask;
     const float om0 = D.om0f;
-    auto cell_index = [&](unsigned l, int& y, int& z) {
+    auto row_of = [&](unsigned l, int& y, int& z) {
       unsigned yq = __umulhi(l + 1u, nz_inv);
-      if (yq * nz > l) --yq;
+      if (yq * nz > l) --yq;  // exact quotient for l < 2^32 / nz - 1
       y = (int)yq + 1;
       z = (int)(l - yq * nz) + 1;
+    };
+    auto cell_index = [&](int x, unsigned l) {
+      int y, z;
+      row_of(l, y, z);
       return (unsigned)sidx(g, x, y, z);
     };
+    auto advance = [&](int& x, unsigned& l, unsigned by) {
+      l += by;
+      while (l >= plane_cells && x <= x1) {
+        l -= plane_cells;
+        x += K;
+      }
+    };
+    int xa = x0, xb;
+    unsigned la = threadIdx.x, lb;
+    advance(xa, la, 0u);
+    xb = xa;
+    lb = la;
+    advance(xb, lb, (unsigned)NT);
     uint2 na = make_uint2(0u, 0u), nb = make_uint2(0u, 0u);
     if (masked) {
-      int y1, z1;
-      if (threadIdx.x < plane_cells) na = batch_links<Q>(D, cell_index(threadIdx.x, y1, z1));
-      if (threadIdx.x + 256u < plane_cells) nb = batch_links<Q>(D, cell_index(threadIdx.x + 256u, y1, z1));
+      if (xa <= x1) na = batch_links<Q>(D, cell_index(xa, la));
+      if (xb <= x1) nb = batch_links<Q>(D, cell_index(xb, lb));
     }
-    for (unsigned l = threadIdx.x; l < plane_cells; l += 512u) {
-      const bool has_b = l + 256u < plane_cells;
-      int ya, za, yb = 0, zb = 0;
-      const unsigned sa = cell_index(l, ya, za);
-      const unsigned sb = has_b ? cell_index(l + 256u, yb, zb) : 0u;
+    while (xa <= x1) {
+      const bool has_b = xb <= x1;
+      const unsigned sa = cell_index(xa, la), sb = has_b ? cell_index(xb, lb) : 0u;
       const uint2 ma = na, mb = nb;
+      const int xa0 = xa, xb0 = xb;
+      const unsigned la0 = la, lb0 = lb;
+      advance(xa, la, 2u * NT);
+      advance(xb, lb, 2u * NT);
       if (masked) {
-        int y1, z1;
-        if (l + 512u < plane_cells) na = batch_links<Q>(D, cell_index(l + 512u, y1, z1));
-        if (l + 768u < plane_cells) nb = batch_links<Q>(D, cell_index(l + 768u, y1, z1));
+        if (xa <= x1) na = batch_links<Q>(D, cell_index(xa, la));
+        if (xb <= x1) nb = batch_links<Q>(D, cell_index(xb, lb));
       }
       int ox[3], oy[3], oz[3];
-      batch_offsets<true>(g, x, ya, za, ox, oy, oz);
+      batch_offsets<true>(g, 0, 0, 0, ox, oy, oz);
       float fa[Q], fb[Q];
       cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, sa, ox, oy, oz, ma.x, fa);
       if (has_b) cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, sb, ox, oy, oz, mb.x, fb);
@@ -212,7 +237,10 @@ __global__ void __launch_bounds__(256, BLOCKS)
       for (int i = 0; i < Q; ++i) f[i] = F2(fa[i], has_b ? fb[i] : 0.f);
       collide_cell<Q, F2, CL_NONE, Store<S>::kDev>(f, p, F2(om0), F2(0.f), rho, u);
       if (p.write_macro) {
-        const long long aa = aidx(g, x, ya, za), ab = aidx(g, x, yb, zb);
+        int ya, za, yb, zb;
+        row_of(la0, ya, za);
+        row_of(lb0, yb, zb);
+        const long long aa = aidx(g, xa0, ya, za), ab = aidx(g, xb0, yb, zb);
         auto put = [&](M* out, F2 v) {
           out[aa] = v.lo();
           if (has_b) out[ab] = v.hi();
@@ -256,11 +284,15 @@ cudaError_t batch_step_shape(const BatchDom* doms, int ndom, const BatchWork& w,
   constexpr int BLOCKS = batch_shape_blocks(SHAPE);
   const int grid = w.grid[BLOCKS - 2], K = w.group[BLOCKS - 2];
   const long long* starts = w.starts + w.off[BLOCKS - 2];
-  auto go = [&](auto kern) { return launch_after(kern, grid, 256, 0, st, doms, ndom, starts, K, p); };
   const bool odd = parity_in == 0;
+  constexpr int NT = batch_shape_threads(SHAPE);
+  auto go = [&](auto kern) { return launch_after(kern, grid, NT, 0, st, doms, ndom, starts, K, p); };
   if constexpr (batch_shape_pair(SHAPE)) {
-    if (odd) return fused ? go(k_batch_step_pair<Q, S, true, true, BLOCKS>) : go(k_batch_step_pair<Q, S, true, false, BLOCKS>);
-    return fused ? go(k_batch_step_pair<Q, S, false, true, BLOCKS>) : go(k_batch_step_pair<Q, S, false, false, BLOCKS>);
+    if (odd)
+      return fused ? go(k_batch_step_pair<Q, S, true, true, BLOCKS, NT>)
+                   : go(k_batch_step_pair<Q, S, true, false, BLOCKS, NT>);
+    return fused ? go(k_batch_step_pair<Q, S, false, true, BLOCKS, NT>)
+                 : go(k_batch_step_pair<Q, S, false, false, BLOCKS, NT>);
   } else {
     if (odd) return fused ? go(k_batch_step<Q, S, true, true, FLAT, BLOCKS>) : go(k_batch_step<Q, S, true, false, FLAT, BLOCKS>);
     return fused ? go(k_batch_step<Q, S, false, true, FLAT, BLOCKS>) : go(k_batch_step<Q, S, false, false, FLAT, BLOCKS>);
