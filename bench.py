@@ -440,9 +440,8 @@ def fd_run(W, w, steps: int, peak: float):
                             "achieved_gbs": gbs, "frac_of_peak": gbs / peak, "steps": steps}
         fd.close()
     out["bytes_per_cell"] = 20
-    out["note"] = ("FP32, velocity read from the LBGK's device field; d3q7: k_fd_step (32 x 8 cell tiles walking 32 "
-                   "x planes); d3q19: k_fd_step_rb (64 x 16 tiles, 4 x 2 cells per thread, a ring of four "
-                   "shared-memory planes, equal runs of planes per resident block)")
+    out["note"] = ("FP32, velocity read from the LBGK's device field; k_fd_march (64 x 8 cell tiles, 64 x 16 for d3q7, "
+                   "marched along x, every plane read once from a ring of three shared-memory planes)")
     del lb, bcs
     return out
 
@@ -768,10 +767,10 @@ def run_ours(args):
     traffic = profile_traffic(f"stream_collide_d3q19_{args.storage}_porous.md", w.cells)
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "peak_source": peak_kind,
-            "kernel": f"k_stream_collide<19,{args.storage}> (AA pattern, odd/even launches averaged)",
+            "kernel": f"k_step_pair<19,{args.storage}> (AA pattern, odd/even launches averaged)",
             "bytes_per_cell": bpc, "cells_per_launch": w.cells, "kernel_ms": tk * 1e3,
-            "note": "algorithmic bytes: read + write of 19 populations per cell; the 8-byte fused-link "
-                    "mask per cell is overhead and not counted"}
+            "note": "algorithmic bytes: read + write of 19 populations per cell; the 4-byte fused-link "
+                    "word per cell is overhead and not counted"}
 
     if rank == 0:
         details = {"separate_conditions": sep, "tma_kernel": direct, "fp16": fp16, "accuracy": accuracy,
