@@ -29,9 +29,12 @@ __host__ __device__ constexpr int batch_shape_blocks(int shape) {
 __host__ __device__ constexpr bool batch_shape_pair(int shape) { return shape >= 3; }
 __host__ __device__ constexpr int batch_shape_threads(int shape) { return shape == 4 ? 320 : 256; }
 
-// A domain's fused-link words of a cell, from its one-word masks where it has them.
-template <int Q>
+// A domain's fused-link words of a cell, from its one-word masks where it has
+// them; FP16 steps are bound by their instructions, not by their bytes, and
+// read the two words (48 channels: 0.263 ms per step, 0.276 with one word).
+template <int Q, class S>
 __device__ __forceinline__ uint2 batch_links(const BatchDom& D, unsigned s) {
+  if (sizeof(S) == 2) return D.mask[s];
   return D.mask32 ? link_words<Q>(D.mask32[s]) : D.mask[s];
 }
 
@@ -130,7 +133,7 @@ __global__ void __launch_bounds__(256, BLOCKS)
     uint2 mnext = make_uint2(0u, 0u);
     if (masked && x <= xb) {
       int y1, z1;
-      mnext = batch_links<Q>(D, cell_index(x, l, y1, z1));
+      mnext = batch_links<Q, S>(D, cell_index(x, l, y1, z1));
     }
     while (x <= xb) {
       int y, z;
@@ -144,7 +147,7 @@ __global__ void __launch_bounds__(256, BLOCKS)
       }
       if (masked && xn <= xb) {
         int y1, z1;
-        mnext = batch_links<Q>(D, cell_index(xn, ln, y1, z1));
+        mnext = batch_links<Q, S>(D, cell_index(xn, ln, y1, z1));
       }
       int ox[3], oy[3], oz[3];
       batch_offsets<FLAT>(g, x, y, z, ox, oy, oz);
@@ -212,8 +215,8 @@ __global__ void __launch_bounds__(NT, BLOCKS)
     advance(xb, lb, (unsigned)NT);
     uint2 na = make_uint2(0u, 0u), nb = make_uint2(0u, 0u);
     if (masked) {
-      if (xa <= x1) na = batch_links<Q>(D, cell_index(xa, la));
-      if (xb <= x1) nb = batch_links<Q>(D, cell_index(xb, lb));
+      if (xa <= x1) na = batch_links<Q, S>(D, cell_index(xa, la));
+      if (xb <= x1) nb = batch_links<Q, S>(D, cell_index(xb, lb));
     }
     while (xa <= x1) {
       const bool has_b = xb <= x1;
@@ -224,8 +227,8 @@ __global__ void __launch_bounds__(NT, BLOCKS)
       advance(xa, la, 2u * NT);
       advance(xb, lb, 2u * NT);
       if (masked) {
-        if (xa <= x1) na = batch_links<Q>(D, cell_index(xa, la));
-        if (xb <= x1) nb = batch_links<Q>(D, cell_index(xb, lb));
+        if (xa <= x1) na = batch_links<Q, S>(D, cell_index(xa, la));
+        if (xb <= x1) nb = batch_links<Q, S>(D, cell_index(xb, lb));
       }
       int ox[3], oy[3], oz[3];
       batch_offsets<true>(g, 0, 0, 0, ox, oy, oz);
