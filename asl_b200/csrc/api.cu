@@ -879,14 +879,19 @@ int build_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key) {
   drop_graph(h);  // it may hold merged launches
   drop_groups(h);
   const int q = h->d.q;
-  auto plain = [&](const aslb_bc* b) { return !b->field() && !b->fused && b->n == 0 && b->nd > 0; };
+  // a condition that stands in the list more than once keeps its own launches:
+  // which of its links a later condition writes differs from place to place,
+  // and the marks are one set per condition
+  auto plain = [&](const aslb_bc* b) {
+    return !b->field() && !b->fused && b->n == 0 && b->nd > 0 && std::count(key.begin(), key.end(), b) == 1;
+  };
   for (size_t i = 0; i < key.size();) {
     LinkGroup g;
     int links = 0;
     size_t j = i, dropped = 0;
     for (; j < key.size() && plain(key[j]) && (long long)links + key[j]->nd <= kGroupLinks; ++j) {
       bool ok = key[j]->bp.scale == key[i]->bp.scale;
-      for (size_t m = i; ok && m < j; ++m) ok = key[m] != key[j] && !conflict(key[m], key[j], q);
+      for (size_t m = i; ok && m < j; ++m) ok = !conflict(key[m], key[j], q);
       int used = 0;
       for (int k = 1; k < q; ++k) used += key[j]->ls.seg[k + 1] > key[j]->ls.seg[k];
       if (!ok || g.segs.n + used > kLinkSegs) break;

@@ -126,6 +126,35 @@ def test_merged_conditions_equal_separate_ones(gpu, storage, case, steps):
     assert_same(out)
 
 
+@pytest.mark.parametrize("storage", ["f32", "f64"])
+@pytest.mark.parametrize("order", ["ABA", "ABAC", "ABCABC", "AfABC", "ABACDBD"])
+def test_lists_that_name_a_condition_twice(gpu, storage, order):
+    """A condition may stand more than once in a list of a run: walls that
+    share edge links (A, B, C, D; the last writer's value stays), and a
+    condition on the density field between them (f)."""
+    shape = (8, 7, 9)
+    g = tuple(s + 2 for s in shape)
+    rho, u = smooth_field(g, 3, amp=0.02)
+    out = []
+    for merged in (True, False):
+        lb = A.LBGK(A.Block(shape), 0.03, A.d3q19(), storage=storage)
+        A.LBGKUtilities(lb).initF(rho, u)
+        bcs = {"A": A.generateBCNoSlip(lb, [A.Y0, A.YE]), "B": A.generateBCConstantVelocity(lb, (0.03, 0.01, 0.0), [A.X0]),
+               "C": A.generateBCConstantPressure(lb, 1.01, [A.XE]),
+               "D": A.generateBCConstantPressureVelocity(lb, 1.02, (0.0, 0.01, 0.0), [A.Z0]),
+               "f": A.generateBCNoSlipRho(lb, sphere_map(g, (4.0, 3.0, 4.0), 1.6))}
+        which = [bcs[k] for k in order]
+        for _ in range(2):  # as recorded first, then replayed
+            if merged:
+                lb.run(6, which)
+            else:
+                for _ in range(6):
+                    lb.execute()
+                    A.executeAll(which)
+        out.append((lb.getF(), lb.getVelocity(), lb.getRho()))
+    assert_same(out)
+
+
 @pytest.mark.parametrize("storage", ["f32", "f16"])
 @pytest.mark.parametrize("q", [15, 19])
 @pytest.mark.parametrize("shape", [3, 4])
