@@ -134,6 +134,7 @@ struct aslb_bc {
   long long links = 0;
   bool fused = false;  // folded into the stream-collide kernel (execute is a no-op)
   BcParams bp{};
+  std::vector<int> marked;         // entries of dlinks that carry kLinkDropped on the device
   std::vector<int> host_links;     // host copies, kept for fusing
   std::vector<int4> host_anchors;
   double* fweights = nullptr;      // field condition on rho: per-cell direction weights
@@ -255,12 +256,10 @@ void drop_graph(aslb_lbgk* h) {
   h->graph_parity = -1;
 }
 
-cudaError_t mark_dropped(aslb_lbgk* h, aslb_bc* bc, const std::vector<int>& at, bool set);
-
-// Forget the merged launches; their conditions (still alive) lose the marks.
+// Forget the merged launches. The marks stay on the conditions' lists, where
+// separate launches ignore them, until build_groups sets those of its own
+// groups: nothing is launched here, whatever the state of the stream.
 void drop_groups(aslb_lbgk* h) {
-  for (LinkGroup& g : h->groups)
-    for (size_t m = 0; m < g.bcs.size(); ++m) mark_dropped(h, g.bcs[m], g.dropped[m], false);
   h->groups.clear();
   h->groups_key.clear();
 }
@@ -864,14 +863,21 @@ bool conflict(const aslb_bc* a, const aslb_bc* b, int q) {
   return false;
 }
 
-cudaError_t mark_dropped(aslb_lbgk* h, aslb_bc* bc, const std::vector<int>& at, bool set) {
+// Make `dropped` the marked links of a condition's list.
+cudaError_t mark_dropped(aslb_lbgk* h, aslb_bc* bc, const std::vector<int>& dropped) {
+  if (bc->marked == dropped) return cudaSuccess;
   cudaError_t e = cudaSuccess;
   LinkMarks m;
-  for (size_t i = 0; e == cudaSuccess && i < at.size(); i += m.n) {
-    m.n = (int)std::min<size_t>(at.size() - i, sizeof(m.at) / sizeof(m.at[0]));
-    std::copy(at.begin() + i, at.begin() + i + m.n, m.at);
-    e = launch_mark_links(bc->dlinks, m, set, h->stream);
-  }
+  auto mark = [&](const std::vector<int>& at, bool set) {
+    for (size_t i = 0; e == cudaSuccess && i < at.size(); i += m.n) {
+      m.n = (int)std::min<size_t>(at.size() - i, sizeof(m.at) / sizeof(m.at[0]));
+      std::copy(at.begin() + i, at.begin() + i + m.n, m.at);
+      e = launch_mark_links(bc->dlinks, m, set, h->stream);
+    }
+  };
+  mark(bc->marked, false);
+  mark(dropped, true);
+  if (e == cudaSuccess) bc->marked = dropped;
   return e;
 }
 
@@ -928,7 +934,7 @@ int build_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key) {
     g.segs.start[g.segs.n] = links;
     h->groups.push_back(g);
     for (size_t m = 0; m < g.bcs.size(); ++m) {
-      cudaError_t e = mark_dropped(h, g.bcs[m], g.dropped[m], true);
+      cudaError_t e = mark_dropped(h, g.bcs[m], g.dropped[m]);
       if (e != cudaSuccess) {
         drop_groups(h);
         return fail(ASLB_ERR_CUDA, std::string("aslb_lbgk_run: ") + cudaGetErrorString(e));
@@ -960,7 +966,7 @@ int aslb_lbgk_run(aslb_lbgk* h, int nsteps, aslb_bc* const* bcs, int nbc, int us
   // a later run with other conditions takes back.
   cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
   if (nbc > 1) ASLB_CUDA(cudaStreamIsCapturing(h->stream, &recording));
-  if (recording == cudaStreamCaptureStatusNone && nsteps >= kGroupSteps && h->groups_key != key) {
+  if (nbc > 1 && recording == cudaStreamCaptureStatusNone && nsteps >= kGroupSteps && h->groups_key != key) {
     int r = build_groups(h, key);
     if (r) return r;
   }

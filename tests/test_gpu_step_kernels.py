@@ -4,6 +4,7 @@ and the separate launches: the same bits (the packed collision rounds each
 cell as the scalar one does, and merging only regroups independent copies)."""
 import numpy as np
 import pytest
+import torch
 
 from asl_b200 import _lib as L
 from asl_b200 import lbgk as A
@@ -151,6 +152,49 @@ def test_lists_that_name_a_condition_twice(gpu, storage, order):
                 for _ in range(6):
                     lb.execute()
                     A.executeAll(which)
+        out.append((lb.getF(), lb.getVelocity(), lb.getRho()))
+    assert_same(out)
+
+
+@pytest.mark.parametrize("recorded", ["walls", "none", "both"])
+def test_merged_conditions_around_a_recording(gpu, recorded):
+    """A run that the caller records on the domain's stream, with one condition,
+    none, or the merged list, leaves the merged launches before and after it,
+    and its own replay, as they are."""
+    shape = (8, 7, 9)
+    rho, u = smooth_field(tuple(s + 2 for s in shape), 3, amp=0.02)
+    out = []
+    for merged in (True, False):
+        lb = A.LBGK(A.Block(shape), 0.03, A.d3q19())
+        A.LBGKUtilities(lb).initF(rho, u)
+        inlet = A.generateBCConstantVelocity(lb, (0.03, 0.01, 0.0), [A.X0])
+        walls = A.generateBCNoSlip(lb, [A.Y0, A.YE, A.Z0, A.ZE])
+        outlet = A.generateBCConstantPressure(lb, 1.01, [A.XE])
+        in_graph = {"walls": [walls], "none": [], "both": [inlet, walls]}[recorded]
+
+        def loop(n, which):
+            for _ in range(n):
+                lb.execute()
+                A.executeAll(which)
+
+        if merged:
+            lb.run(8, [inlet, walls])
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.stream(torch.cuda.ExternalStream(lb.stream)):
+                graph.capture_begin(capture_error_mode="thread_local")
+                lb.run(4, in_graph, use_graph=False)
+                graph.capture_end()
+            lb.run(8, [inlet, outlet])
+            with torch.cuda.stream(torch.cuda.ExternalStream(lb.stream)):
+                graph.replay()
+            lb.run(8, [inlet, outlet])
+            lb.run(5, [inlet, walls])
+        else:
+            loop(8, [inlet, walls])
+            loop(8, [inlet, outlet])
+            loop(4, in_graph)
+            loop(8, [inlet, outlet])
+            loop(5, [inlet, walls])
         out.append((lb.getF(), lb.getVelocity(), lb.getRho()))
     assert_same(out)
 
