@@ -2,6 +2,7 @@
 // construction of the compact boundary-link lists, and the time loop.
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -82,10 +83,14 @@ struct aslb_lbgk {
   int graph_steps = 0;
   long long graph_version = -1;
   long long version = 0;  // bumped by every parameter change
-  // conditions of the time loop that run as one launch (build_groups), for
+  // conditions of the time loop that run as one launch (update_groups), for
   // the condition list they were built for
   std::vector<LinkGroup> groups;
   std::vector<aslb_bc*> groups_key;
+  // the condition list of the last run, how many runs and steps in a row have
+  // had it, and the steps from which another check is worth it
+  std::vector<aslb_bc*> run_key;
+  long long run_count = 0, run_steps = 0, run_try = 0;
   // fused no-slip conditions
   // fresh: populations were (re)initialised and no fused condition has run
   // since, so incoming slots still hold their initial values and the next
@@ -257,11 +262,12 @@ void drop_graph(aslb_lbgk* h) {
 }
 
 // Forget the merged launches. The marks stay on the conditions' lists, where
-// separate launches ignore them, until build_groups sets those of its own
+// separate launches ignore them, until update_groups sets those of its own
 // groups: nothing is launched here, whatever the state of the stream.
 void drop_groups(aslb_lbgk* h) {
   h->groups.clear();
   h->groups_key.clear();
+  h->run_key.clear();  // the address of a destroyed condition may come back
 }
 
 template <class T>
@@ -814,12 +820,21 @@ namespace {
 // direction-sorted conditions can run as one when no link of one reads a slot
 // that a link of another writes, in either representation; a link that a later
 // condition writes too is left to that one (ASL's order: the last writer
-// wins). Above kGroupLinks links a launch is no longer what costs. The check
-// and the marks take some tens of microseconds once per condition list, and
-// nothing is allocated: the launch reads the conditions' own lists.
+// wins). Above kGroupLinks links a launch is no longer what costs. Nothing is
+// allocated: the launch reads the conditions' own lists. The check walks the
+// sorted lists on the host where their index ranges overlap, 0.8 to 1.7 ns per
+// entry: 25 us for the four walls, inlet and outlet of a 128x64x64 channel
+// (204,288 links), 2.1 ms with the 254,883 links of a porous map in it, where
+// merging saves 5 us per step. So a list is checked once its steps in a row
+// would have paid for the walk (kGroupWalk entries per step and launch saved),
+// and takes the place of another list's launches only in its second run in a
+// row or in a long one: a program that alternates between lists keeps the
+// launches of the first (64x32x32 porous channel, two lists in turn, runs of
+// four steps: 0.34 ms per pair of runs, 0.98 when every run merged its own).
 constexpr long long kGroupLinks = 1 << 20;
 constexpr size_t kGroupDropped = 16384;
-constexpr int kGroupSteps = 4;
+constexpr int kGroupSteps = 4, kGroupLongRun = 32;
+constexpr long long kGroupWalk = 1000;
 
 struct LinkRange {  // ascending storage indices, all displaced by off
   const int* p;
@@ -836,9 +851,11 @@ LinkRange outgoing(const aslb_bc* b, int k) {  // direction inv k at the fluid e
 }
 // Calls f(index in a, index in b) for every common index of two ranges until f
 // returns true; true then. Only the part of each range inside the other's is
-// walked (a wall's links lie in one plane of a channel).
+// walked (a wall's links lie in one plane of a channel), and what is walked is
+// taken off `walk`; below zero nothing is walked any more and the answer means
+// nothing.
 template <class F>
-bool common(const LinkRange& a, const LinkRange& b, F f) {
+bool common(const LinkRange& a, const LinkRange& b, long long& walk, F f) {
   if (a.p == a.e || b.p == b.e) return false;
   const int lo = std::max(a.p[0] + a.off, b.p[0] + b.off), hi = std::min(a.e[-1] + a.off, b.e[-1] + b.off);
   if (lo > hi) return false;
@@ -846,6 +863,8 @@ bool common(const LinkRange& a, const LinkRange& b, F f) {
   const int* j = std::lower_bound(b.p, b.e, lo - b.off);
   const int* ie = std::upper_bound(i, a.e, hi - a.off);
   const int* je = std::upper_bound(j, b.e, hi - b.off);
+  walk -= (ie - i) + (je - j);
+  if (walk < 0) return false;
   while (i != ie && j != je) {
     const int d = (*i + a.off) - (*j + b.off);
     if (d == 0 && f(i - a.p, j - b.p)) return true;
@@ -854,11 +873,11 @@ bool common(const LinkRange& a, const LinkRange& b, F f) {
   }
   return false;
 }
-bool conflict(const aslb_bc* a, const aslb_bc* b, int q) {
+bool conflict(const aslb_bc* a, const aslb_bc* b, int q, long long& walk) {
   auto yes = [](long long, long long) { return true; };
   for (int k = 1; k < q; ++k) {
     const int j = a->ls.inv[k];
-    if (common(outgoing(a, k), incoming(b, j), yes) || common(incoming(a, j), outgoing(b, k), yes)) return true;
+    if (common(outgoing(a, k), incoming(b, j), walk, yes) || common(incoming(a, j), outgoing(b, k), walk, yes)) return true;
   }
   return false;
 }
@@ -881,9 +900,9 @@ cudaError_t mark_dropped(aslb_lbgk* h, aslb_bc* bc, const std::vector<int>& drop
   return e;
 }
 
-int build_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key) {
-  drop_graph(h);  // it may hold merged launches
-  drop_groups(h);
+// The merged launches of a condition list. Gives up (false) when the check
+// walks more than `walk` list entries; sets nothing on the device.
+bool find_groups(const aslb_lbgk* h, const std::vector<aslb_bc*>& key, long long walk, std::vector<LinkGroup>& out) {
   const int q = h->d.q;
   // a condition that stands in the list more than once keeps its own launches:
   // which of its links a later condition writes differs from place to place,
@@ -897,7 +916,7 @@ int build_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key) {
     size_t j = i, dropped = 0;
     for (; j < key.size() && plain(key[j]) && (long long)links + key[j]->nd <= kGroupLinks; ++j) {
       bool ok = key[j]->bp.scale == key[i]->bp.scale;
-      for (size_t m = i; ok && m < j; ++m) ok = !conflict(key[m], key[j], q);
+      for (size_t m = i; ok && m < j; ++m) ok = !conflict(key[m], key[j], q, walk);
       int used = 0;
       for (int k = 1; k < q; ++k) used += key[j]->ls.seg[k + 1] > key[j]->ls.seg[k];
       if (!ok || g.segs.n + used > kLinkSegs) break;
@@ -917,7 +936,7 @@ int build_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key) {
         g.segs.vald[s] = b->ls.vald[k];
         // links that this condition writes after an earlier one
         for (size_t m = 0; m < g.bcs.size(); ++m)
-          common(incoming(g.bcs[m], k), incoming(b, k), [&](long long x, long long) {
+          common(incoming(g.bcs[m], k), incoming(b, k), walk, [&](long long x, long long) {
             g.dropped[m].push_back(g.bcs[m]->ls.seg[k] + (int)x);
             ++dropped;
             return false;
@@ -927,12 +946,38 @@ int build_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key) {
       g.bcs.push_back(b);
       g.dropped.emplace_back();
     }
+    if (walk < 0) return false;
     if (g.bcs.size() < 2 || dropped > kGroupDropped) {
       ++i;
       continue;
     }
     g.segs.start[g.segs.n] = links;
-    h->groups.push_back(g);
+    out.push_back(g);
+    i = j;
+  }
+  return true;
+}
+
+// Called by every run that is not recorded, before its first step: counts the
+// runs of a list and merges its conditions when that pays (see above).
+int update_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key, int nsteps) {
+  if (h->run_key != key) {
+    h->run_key = key;
+    h->run_count = h->run_steps = h->run_try = 0;
+  }
+  h->run_count += 1;
+  h->run_steps += nsteps;
+  if (key.size() < 2 || nsteps < kGroupSteps || h->groups_key == key || h->run_steps < h->run_try) return ASLB_OK;
+  if (!h->groups.empty() && h->run_count < 2 && nsteps < kGroupLongRun) return ASLB_OK;
+  std::vector<LinkGroup> found;
+  if (!find_groups(h, key, h->run_steps * kGroupWalk * (long long)(key.size() - 1), found)) {
+    h->run_try = 2 * h->run_steps;
+    return ASLB_OK;
+  }
+  h->run_try = LLONG_MAX;  // found for good, or there are none
+  if (found.empty()) return ASLB_OK;
+  drop_graph(h);  // it may hold merged launches
+  for (LinkGroup& g : found)
     for (size_t m = 0; m < g.bcs.size(); ++m) {
       cudaError_t e = mark_dropped(h, g.bcs[m], g.dropped[m]);
       if (e != cudaSuccess) {
@@ -940,8 +985,7 @@ int build_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key) {
         return fail(ASLB_ERR_CUDA, std::string("aslb_lbgk_run: ") + cudaGetErrorString(e));
       }
     }
-    i = j;
-  }
+  h->groups = std::move(found);
   h->groups_key = key;
   return ASLB_OK;
 }
@@ -966,8 +1010,8 @@ int aslb_lbgk_run(aslb_lbgk* h, int nsteps, aslb_bc* const* bcs, int nbc, int us
   // a later run with other conditions takes back.
   cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
   if (nbc > 1) ASLB_CUDA(cudaStreamIsCapturing(h->stream, &recording));
-  if (nbc > 1 && recording == cudaStreamCaptureStatusNone && nsteps >= kGroupSteps && h->groups_key != key) {
-    int r = build_groups(h, key);
+  if (recording == cudaStreamCaptureStatusNone) {
+    int r = update_groups(h, key, nsteps);
     if (r) return r;
   }
   const std::vector<LinkGroup>* groups =

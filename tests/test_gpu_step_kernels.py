@@ -92,7 +92,8 @@ def test_merged_conditions_equal_separate_ones(gpu, storage, case, steps):
     """run() of 4 steps or more merges consecutive conditions (and of 32 or more
     replays eight steps at a time); walls share edge links (the later
     condition's value stays), and two maps whose links read each other's slots
-    are left separate."""
+    are left separate. Lists in turn, lists that take another's place, and
+    lists after a condition was destroyed."""
     shape = (14, 10, 9)
     g = tuple(s + 2 for s in shape)
     rho, u = smooth_field(g, 11, amp=0.02)
@@ -111,19 +112,23 @@ def test_merged_conditions_equal_separate_ones(gpu, storage, case, steps):
         elif case == "fused_last":
             bcs.append(A.generateBCNoSlip(lb, sphere_map(g, (6.0, 5.0, 4.0), 2.6)))
             bcs[-1].fuse()
-        # the same list twice, then others (merged again or dropped), then back
-        for which in (bcs, bcs, bcs[:2], [bcs[0], *bcs[2:]], bcs):
+
+        def go(which):
             if merged:
                 lb.run(steps, which)
             else:
                 for _ in range(steps):
                     lb.execute()
                     A.executeAll(which)
+
+        # the same list twice, another in turn with it, then others in its place, then back
+        others = [[bcs[0], *bcs[2:]], bcs[:2], [bcs[2], bcs[0], *bcs[3:]]]
+        for which in (bcs, bcs, others[1], bcs, others[0], others[0], others[1], others[1], others[2], others[2], bcs, bcs):
+            go(which)
+        del bcs[1], which, others
+        go(bcs)
+        go(bcs)
         out.append((lb.getF(), lb.getVelocity(), lb.getRho()))
-        if merged:  # a destroyed condition
-            del bcs[1], which
-            lb.run(steps, bcs)
-            lb.sync()
     assert_same(out)
 
 
