@@ -208,7 +208,10 @@ __global__ void __launch_bounds__(kFdTZ * kFdTY) k_fd_step(const T* __restrict__
 // three slots, two planes ahead of the arithmetic, without registers.
 // Work: items of `len` planes of a tile, all tiles of an x range before the
 // next range, so that the blocks running together share their tiles' halo
-// rows in L2 (tile by tile, the halos come from HBM again).
+// rows in L2 (tile by tile, the halos come from HBM again). Element indices are
+// 32-bit: blocks of 2^32 cells or more take k_fd_step (with a 64-bit pointer per
+// plane and field d3q19 took 0.0643 ms per step at 256x192x192 instead of
+// 0.0618).
 // KY: two, four for d3q7, whose cells carry fewer sums (512x256x256 FP32 with
 // velocity, ms per step with two / four: d3q7 0.187 / 0.183, 0.062 / 0.049 at
 // 256x192x192; d3q19 0.215 / 0.243).
@@ -276,7 +279,7 @@ __global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
   wait_before();
   let_next();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned plane = (unsigned)(g.gy * g.gz);
+  const unsigned plane = (unsigned)g.gy * (unsigned)g.gz;
   const F2 a = F2(ga), d = F2(gd), D = F2(Df), half = F2(0.5f), two = F2(2.f);
   for (int item = blockIdx.x; item < items; item += gridDim.x) {
     const int tile = item % tiles;
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
     for (int k = 0; k < R::E; ++k) {
       const int e = (int)threadIdx.x + k * NT;
       const int yy = y0 + e / W, zz = z0 + e % W;
-      off[k] = (e < P && yy < g.gy && zz < g.gz) ? (unsigned)(yy * g.gz + zz) : ~0u;
+      off[k] = (e < P && yy < g.gy && zz < g.gz) ? (unsigned)yy * (unsigned)g.gz + (unsigned)zz : ~0u;
     }
     auto fetch = [&](int xp) {
       if (xp <= xb + 1) {
@@ -371,7 +374,7 @@ __global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
           }
           const int y = y1 + r;
           if (y <= g.ny) {
-            float* out = cn + (size_t)((unsigned)(x - 1) * plane + (unsigned)(y * g.gz + z));
+            float* out = cn + (size_t)((unsigned)(x - 1) * plane + (unsigned)y * (unsigned)g.gz + (unsigned)z);
             if (z <= g.nz) out[0] = o.lo();
             if (z < g.nz) out[1] = o.hi();
           }
@@ -574,10 +577,11 @@ cudaError_t fd_launch_march(aslb_fd* f) {
 
 template <int Q, class T>
 cudaError_t fd_launch(aslb_fd* f) {
-  // FP32 without the electric term: the marching kernel; FP64 (whose sums
-  // would take twice the registers) and the electric term: the 32 x 8 tiles
+  // FP32 without the electric term: the marching kernel, within its 32-bit
+  // element indices; FP64 (whose sums would take twice the registers), the
+  // electric term and larger blocks: the 32 x 8 tiles
   if constexpr (std::is_same<T, float>::value) {
-    if (!f->ef) {
+    if (!f->ef && f->g.L < (1LL << 32)) {
       if (!f->u) return fd_launch_march<Q, false, false>(f);
       return f->cc ? fd_launch_march<Q, true, true>(f) : fd_launch_march<Q, true, false>(f);
     }

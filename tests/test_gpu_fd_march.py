@@ -1,9 +1,13 @@
 """The marching FD step at the edges of its tiles (64 z, 8 or 16 y cells) and
 items (runs of x planes), against the numpy oracle in double precision."""
+import ctypes as C
+
 import numpy as np
 import pytest
+import torch
 
 from asl_b200 import fd as FD
+from asl_b200 import _lib as L
 from asl_b200 import lbgk as A
 from oracle.fd_oracle import fd_step
 
@@ -29,3 +33,41 @@ def test_tile_edges_match_oracle(gpu, q, cc, shape):
         # three steps of about 60 FP32 operations on values up to 1.2 (a
         # rounding is 6e-8 of its size, the products are a tenth of c)
         assert np.abs(fd.getC() - ref).max() < 2e-6
+
+
+class Field:
+    """Device memory of the solver as an array that torch reads in place."""
+
+    def __init__(self, pointer, shape):
+        self.__cuda_array_interface__ = dict(shape=shape, typestr="<f4", data=(pointer, False), version=2)
+
+
+@pytest.mark.parametrize("q", [7, 15, 19])
+def test_more_than_2_to_32_cells(gpu, q):
+    """A block whose element indices do not fit 32 bits (two fields of 17.3 GB):
+    random planes at both ends and around 2^32 cells, zero elsewhere."""
+    gx, gy, gz = 4120, 1030, 1020
+    per_plane = gy * gz
+    assert gx * per_plane > 2**32 + 20 * per_plane
+    lib, h = L.load(), C.c_void_p()
+    L.check(lib.aslb_fd_create(gx - 2, gy - 2, gz - 2, q, L.F32, 0.07, C.byref(h)))
+    try:
+        field = torch.as_tensor(Field(lib.aslb_fd_device_field(h), (gx, gy, gz)), device="cuda")
+        rng = np.random.default_rng(q)
+        blocks = [0, 2**32 // per_plane - 3, gx - 7]  # first planes of seven each
+        part = {x: rng.uniform(0.2, 1.2, (7, gy, gz)).astype(np.float32) for x in blocks}
+        for x, v in part.items():
+            field[x:x + 7] = torch.from_numpy(v).cuda()
+        torch.cuda.synchronize()
+        L.check(lib.aslb_fd_step(h, 1))
+        L.check(lib.aslb_fd_sync(h))
+        out = torch.as_tensor(Field(lib.aslb_fd_device_field(h), (gx, gy, gz)), device="cuda")
+        for x, v in part.items():
+            got = out[x + 1:x + 6, 1:-1, 1:-1].cpu().numpy()
+            # 20 FP32 operations on values up to 1.2 (a rounding is 6e-8 of its size)
+            assert np.abs(got - fd_step(v.astype(np.float64), 0.07, q, None, False)[1:-1, 1:-1, 1:-1]).max() < 2e-6
+        # planes whose neighbours are zero too
+        for x in (9, blocks[1] // 2, blocks[1] - 3, blocks[1] + 9, gx - 10):
+            assert not out[x, 1:-1, 1:-1].any()
+    finally:
+        lib.aslb_fd_destroy(h)
