@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
   let_next();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned plane = (unsigned)g.gy * (unsigned)g.gz;
-  const F2 a = F2(ga), d = F2(gd), D = F2(Df), half = F2(0.5f), two = F2(2.f);
+  const F2 a = F2(ga), d = F2(gd), D = F2(Df), half = F2(0.5f), mhalf = F2(-0.5f), two = F2(2.f);
   for (int item = blockIdx.x; item < items; item += gridDim.x) {
     const int tile = item % tiles;
     const int xa = (item / tiles) * len + 1, xb = min(g.nx, xa + len - 1);
@@ -311,8 +311,11 @@ __global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int z = z0 + 2 * lane + 1, y1 = y0 + w * KY + 1;
-    // outputs of the previous plane, up to that plane's own sums (acc: with
-    // the correction without div and lap, which cl and cd hold), and its centre
+    // the previous plane's outputs less its centre, up to that plane's own
+    // sums (with the correction cl and cd hold lap and div), and its centre
+    // (cc, cu, cv, cw). The centre is added last, in one rounding of its size:
+    // with the centre in acc from the start, three such roundings put a step
+    // a fifth farther from the sums in double precision
     F2 acc[KY], cl[KY], cd[KY], cc[KY], cu[KY], cv[KY], cw[KY];
     // the current plane's sums for the next plane's outputs
     F2 sX[KY], sU[KY], sP[KY], sY[KY], sZ[KY];
@@ -359,18 +362,19 @@ __global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
         }
         if (x > xa) {
           // outputs of plane x - 1: this plane's share
-          F2 o = fma_(mul_(two, D), X, acc[r]);
+          F2 o = fma_(mul_(two, D), X, acc[r]), B;
           if constexpr (U) {
-            const F2 B = add_(Tu, Xu);
+            B = add_(Tu, Xu);
             F2 f = fma_(cc[r], B, add_(Tp_, Xp));
             f = fma_(cu[r], X, f);
             if (Q > 7) f = fma_(cw[r], Gz, fma_(cv[r], Gy, f));
-            o = sub_(o, mul_(half, f));
-            if constexpr (CC) {
-              o = div_(o, sub_(F2(1.f), add_(cd[r], B)));
-              const F2 uu = fma_(cw[r], cw[r], fma_(cv[r], cv[r], mul_(cu[r], cu[r])));
-              o = fma_(fma_(two, X, cl[r]), mul_(uu, half), o);
-            }
+            o = fma_(mhalf, f, o);
+          }
+          o = add_(cc[r], o);
+          if constexpr (CC) {
+            o = div_(o, sub_(F2(1.f), add_(cd[r], B)));
+            const F2 uu = fma_(cw[r], cw[r], fma_(cv[r], cv[r], mul_(cu[r], cu[r])));
+            o = fma_(fma_(two, X, cl[r]), mul_(uu, half), o);
           }
           const int y = y1 + r;
           if (y <= g.ny) {
@@ -384,7 +388,8 @@ __global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
           F2 L = fma_(F2((float)Tp::lc(0)), mid.cm, mul_(mul_(two, a), cross));
           if (Q == 19) L = fma_(mul_(two, d), corner, L);
           L = fma_(two, sX[r], L);
-          F2 o = fma_(D, L, mid.cm);
+          F2 o = mul_(D, L);
+          cc[r] = mid.cm;
           if constexpr (U) {
             F2 By = fma_(a, q1, sP[r]), Bu = fma_(a, v1, sU[r]);
             F2 gy = mul_(a, dy), gz = mul_(a, mid.cd);
@@ -401,8 +406,7 @@ __global__ void __launch_bounds__(MarchConf<Q>::NT, 2)
             F2 f = fma_(mid.cm, Bu, By);
             f = fma_(mid.vm, gy, sub_(f, mul_(mid.um, sX[r])));
             f = fma_(mid.wm, gz, f);
-            o = sub_(o, mul_(half, f));
-            cc[r] = mid.cm;
+            o = fma_(mhalf, f, o);
             cu[r] = mid.um;
             cv[r] = mid.vm;
             cw[r] = mid.wm;

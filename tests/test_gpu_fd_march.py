@@ -71,3 +71,24 @@ def test_more_than_2_to_32_cells(gpu, q):
             assert not out[x, 1:-1, 1:-1].any()
     finally:
         lib.aslb_fd_destroy(h)
+
+
+@pytest.mark.parametrize("q", [7, 15, 19])
+@pytest.mark.parametrize("flow", [False, True])
+def test_one_rounding_of_the_centre(gpu, q, flow):
+    """A step adds its increment to the centre once. Values in [1, 2) round with
+    a root mean square of 2^-23 / sqrt(12); the increment is a twentieth of
+    them or less and its dozen roundings add a tenth of that, a second rounding
+    of the sum would add 40 %."""
+    shape = (20, 34, 66)
+    g = tuple(s + 2 for s in shape)
+    rng = np.random.default_rng(q)
+    c = rng.uniform(1.4, 1.6, g).astype(np.float32)
+    u = rng.uniform(-0.05, 0.05, (3, *g)).astype(np.float32)
+    lb = A.LBGK(A.Block(shape), 0.05, A.d3q19())
+    A.LBGKUtilities(lb).initF(u.astype(np.float64))
+    fd = FD.generateFDAdvectionDiffusion(c, 0.01, lb if flow else None, q, False)
+    fd.execute()
+    want = fd_step(c.astype(np.float64), np.float64(np.float32(0.01)), q, u.astype(np.float64) if flow else None, False)
+    err = (fd.getC() - want)[1:-1, 1:-1, 1:-1]
+    assert np.sqrt((err**2).mean()) < 1.2 * 2.0**-23 / np.sqrt(12)
