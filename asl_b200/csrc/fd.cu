@@ -28,6 +28,7 @@
 #include "f32x2.cuh"
 #include "lattice.cuh"
 #include "launch.cuh"
+#include "per_device.h"
 #include "tma.cuh"
 
 namespace aslb {
@@ -533,16 +534,21 @@ int fd_arg(const char* what) {
 size_t fd_elem(const aslb_fd* f) { return f->dtype == ASLB_F64 ? 8 : 4; }
 
 // Launch one instantiation with its dynamic shared memory (three tile planes
-// of every field it stages), raising the limit once where above 48 KB.
+// of every field it stages), raising the device's limit where above 48 KB.
 template <int Q, class T, bool U, bool E>
 cudaError_t fd_launch_one(aslb_fd* f, dim3 grid, dim3 block, const T* c, T* cn, const T* u, const T* ef) {
   constexpr int NF = 1 + (U ? 3 : 0) + (E ? 3 : 0);
   constexpr size_t bytes = 3u * NF * (kFdTZ + 2) * (kFdTY + 2) * sizeof(T);
-  static bool raised = false;
-  if (bytes > 48 * 1024 && !raised) {
-    cudaError_t e = cudaFuncSetAttribute(k_fd_step<Q, T, U, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (bytes > 48 * 1024) {
+    static PerDevice raised;
+    int dev = 0, limit = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+      e = raised.get(dev, limit, [&](int& n) {
+        n = (int)bytes;
+        return cudaFuncSetAttribute(k_fd_step<Q, T, U, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
+      });
     if (e != cudaSuccess) return e;
-    raised = true;
   }
   return launch_after(k_fd_step<Q, T, U, E>, grid, block, bytes, f->stream, c, cn, u, ef, f->g, T(f->D), U ? f->cc : 0);
 }
@@ -553,17 +559,15 @@ cudaError_t fd_launch_march(aslb_fd* f) {
   using R = MarchConf<Q>;
   constexpr size_t bytes = fd_march_smem<Q, U>();
   auto kern = k_fd_march<Q, U, CC>;
-  static int resident = 0;  // blocks per SM
-  if (!resident) {
-    int n = 0;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, R::NT, bytes);
-    if (e != cudaSuccess) return e;
-    if (n < 1) return cudaErrorInvalidConfiguration;
-    resident = n;
-  }
-  int dev = 0, sms = 0;
+  static PerDevice blocks;
+  int dev = 0, sms = 0, resident = 0;  // blocks per SM
   cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = blocks.get(dev, resident, [&](int& n) {
+      cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      if (r == cudaSuccess) r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, R::NT, bytes);
+      return r == cudaSuccess && n < 1 ? cudaErrorInvalidConfiguration : r;
+    });
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   const int ntz = (f->g.nz + R::TZ - 1) / R::TZ, nty = (f->g.ny + R::TY * R::KY - 1) / (R::TY * R::KY);

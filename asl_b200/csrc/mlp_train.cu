@@ -21,6 +21,7 @@
 #include "f32x2.cuh"
 #include "kernels.h"
 #include "mlp.cuh"
+#include "per_device.h"
 
 namespace aslb {
 
@@ -341,18 +342,21 @@ size_t aslb_mlp_grad_scratch_floats(void) { return (size_t)kGradBlocks * (kParam
 int aslb_mlp_grad(const float* params, const float* x, const float* t, long long n, const float* norm,
                   float out_scale, float* scratch, float* grad_loss, void* stream) {
   if (!params || !x || !t || !norm || !scratch || !grad_loss || n <= 0) return arg_err("aslb_mlp_grad");
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grad_smem());
-    if (e != cudaSuccess) return err("aslb_mlp_grad", e);
-    configured = true;
-  }
+  static PerDevice configured;
+  int dev = 0, limit = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = configured.get(dev, limit, [](int& n) {
+      n = (int)grad_smem();
+      return cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
+    });
+  if (e != cudaSuccess) return err("aslb_mlp_grad", e);
   cudaStream_t st = (cudaStream_t)stream;
   const long long chunks = (n + kChunk - 1) / kChunk;
   const int blocks = (int)(chunks < kGradBlocks ? chunks : kGradBlocks);
   k_mlp_grad<<<blocks, kGradThreads, grad_smem(), st>>>(params, x, t, n, norm, out_scale, 1.f / (float)n, scratch);
   k_mlp_reduce<<<(kParams + kReduceCols) / kReduceCols, kReduceCols * kReduceWays, 0, st>>>(scratch, blocks, grad_loss);
-  const cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   return e == cudaSuccess ? ASLB_OK : err("aslb_mlp_grad", e);
 }
 
@@ -389,4 +393,3 @@ int aslb_mlp_pack(const float* params_host, const float* norm_host, float out_sc
 }
 
 }  // extern "C"
-

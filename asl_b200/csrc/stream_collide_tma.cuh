@@ -16,6 +16,7 @@
 // upstream cell falls outside the segment reads it from global memory.
 #pragma once
 #include "stream_collide.cuh"
+#include "per_device.h"
 #include "tma.cuh"
 #include <algorithm>
 
@@ -238,21 +239,16 @@ cudaError_t step_tma(const DomainDev& d, const StepParams& p, int parity_in, cud
   constexpr int target = TmaOccupancy<S, CL>::blocks;
   const TmaShape sh = tma_shape<Q, S>(d.g, p.mask != nullptr, target);
   const size_t smem = (size_t)sh.stages * sh.stage_bytes;
-  static int sm_count = 0;
-  static bool configured[2] = {false, false};
-  if (!sm_count) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-  }
+  static PerDevice configured[2];
+  int dev = 0, sm_count = 0, per_sm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   auto kern = parity_in == 0 ? k_stream_collide_tma<Q, S, CL, true> : k_stream_collide_tma<Q, S, CL, false>;
-  if (!configured[parity_in]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return e;
-    configured[parity_in] = true;
-  }
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTmaThreads, smem);
+  if (e == cudaSuccess)
+    e = configured[parity_in].get(dev, sm_count, [&](int& n) {
+      cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      return r == cudaSuccess ? cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) : r;
+    });
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTmaThreads, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   const int grid = std::min(sh.ntiles, sm_count * per_sm);

@@ -71,3 +71,12 @@ def test_argument_errors_without_gpu(lib):
     assert lib.aslb_lbgk_create(4, 4, 4, 19, 0, -0.1, 0, ctypes.byref(h)) != 0
     assert lib.aslb_bc_execute(None) != 0
     assert lib.aslb_mlp_layout_bytes() > 0
+
+
+def test_launch_settings_are_kept_per_device(tmp_path):
+    """A kernel's shared-memory limit and residency belong to a device: what is
+    found on one is not used on another, and an error is not kept."""
+    src, exe = ROOT / "tests" / "cpp" / "per_device.cc", tmp_path / "per_device"
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", str(ROOT / "asl_b200" / "csrc"), str(src), "-o", str(exe)],
+                   check=True)
+    assert subprocess.run([str(exe)], capture_output=True, text=True).stdout == "ok\n"
