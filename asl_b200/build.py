@@ -31,7 +31,8 @@ def nvcc() -> str:
 
 
 def _sources() -> list[Path]:
-    return sorted(CSRC.glob("*.cu"))
+    """The longest compilations first (two to four minutes each for D3Q27 and D3Q19)."""
+    return sorted(CSRC.glob("*.cu"), key=lambda p: ("_q27_" not in p.name, "_q19_" not in p.name, p.name))
 
 
 def _headers() -> list[Path]:

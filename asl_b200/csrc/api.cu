@@ -99,6 +99,7 @@ struct aslb_lbgk {
   std::vector<uint2> mask_host;
   uint2* mask_dev = nullptr;
   uint32_t* mask32_dev = nullptr;  // the same in one word per cell, where they fit (link_words)
+  bool mask32_single = true;       // no cell of mask32_dev has both kinds of links
   // conditions and force objects made on this domain; destroying the domain
   // releases their device memory and detaches them (any destruction order)
   std::vector<aslb_bc*> bcs;
@@ -1687,11 +1688,15 @@ int aslb_bc_fuse(aslb_bc* bc) {
     out = kBothLinks | faces << 18 | w.y >> 1;
     return q < 27 && all == w.x;
   };
-  bool compact = true;
+  bool compact = true, single = true;
   std::vector<uint32_t> m32(m.size());
-  for (size_t i = 0; compact && i < m.size(); ++i) compact = one_word(m[i], m32[i]);
+  for (size_t i = 0; compact && i < m.size(); ++i) {
+    compact = one_word(m[i], m32[i]);
+    single &= !(m[i].x && m[i].y);
+  }
   cudaFree(h->mask32_dev);
   h->mask32_dev = nullptr;
+  h->mask32_single = single;
   if (compact) {
     ASLB_CUDA(cudaMalloc((void**)&h->mask32_dev, ((size_t)g.dstride + 4096) * sizeof(uint32_t)));
     ASLB_CUDA(cudaMemcpy(h->mask32_dev, m32.data(), m32.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -1946,7 +1951,7 @@ struct aslb_batch {
   long long ntiles = 0;
   long long* dev_starts = nullptr;  // the work split's run tables (BatchWork)
   BatchWork work{};
-  bool any_mask = false;
+  int links = kLinksNone;  // BatchLinks
   std::vector<BatchBc*> dev_pos;  // one table per condition position
   std::vector<int> pos_n;
   std::vector<long long> pos_links;
@@ -2005,7 +2010,7 @@ int batch_tables(aslb_batch* b, aslb_bc* const* bcs, const int* nbc) {
   const int n = (int)b->doms.size();
   b->host_doms.assign(n, BatchDom{});
   b->ntiles = 0;
-  b->any_mask = false;
+  b->links = kLinksNone;
   for (int i = 0; i < n; ++i) {
     aslb_lbgk* h = b->doms[i];
     BatchDom& D = b->host_doms[i];
@@ -2014,7 +2019,7 @@ int batch_tables(aslb_batch* b, aslb_bc* const* bcs, const int* nbc) {
     D.F = h->d.F;
     D.mask = h->fresh ? nullptr : h->mask_dev;
     D.mask32 = h->fresh ? nullptr : h->mask32_dev;
-    b->any_mask |= D.mask != nullptr;
+    if (D.mask && b->links != kLinksBoth) b->links = D.mask32 && h->mask32_single ? kLinksSingle : kLinksBoth;
     b->work.periodic |= g.periodic != 0;
     D.rho = h->d.rho;
     D.u = h->d.u;
@@ -2092,7 +2097,7 @@ int batch_step(aslb_batch* b) {
   aslb_lbgk* h0 = b->doms[0];
   prepare_params(h0);
   const int parity = h0->parity;
-  cudaError_t e = launch_batch_step(b->q, b->storage, b->dev_doms, (int)b->doms.size(), b->work, b->any_mask,
+  cudaError_t e = launch_batch_step(b->q, b->storage, b->dev_doms, (int)b->doms.size(), b->work, b->links,
                                     h0->p, parity, b->shape, b->stream);
   for (size_t j = 0; e == cudaSuccess && j < b->dev_pos.size(); ++j)
     if (b->pos_n[j] > 0)

@@ -1,19 +1,38 @@
-// Dispatch of the batched step and links to their per-storage instantiations
-// (batch_f32.cu, batch_f16.cu, batch_f64.cu; kernels in batch.cuh).
+// Dispatch of the batched step and links to their instantiations per lattice
+// and storage (batch_q15_f32.cu, ...; kernels in batch.cuh).
 #include <algorithm>
 #include "kernels.h"
 
 namespace aslb {
 
-cudaError_t batch_step_f32(int q, const BatchDom* doms, int ndom, const BatchWork& w, int fused, const StepParams& p,
-                           int parity_in, int shape, cudaStream_t st);
-cudaError_t batch_step_f16(int q, const BatchDom* doms, int ndom, const BatchWork& w, int fused, const StepParams& p,
-                           int parity_in, int shape, cudaStream_t st);
-cudaError_t batch_step_f64(int q, const BatchDom* doms, int ndom, const BatchWork& w, int fused, const StepParams& p,
-                           int parity_in, int shape, cudaStream_t st);
-cudaError_t batch_links_f32(int q, const BatchBc* bcs, int nbc, long long nlinks, int parity, cudaStream_t st);
-cudaError_t batch_links_f16(int q, const BatchBc* bcs, int nbc, long long nlinks, int parity, cudaStream_t st);
-cudaError_t batch_links_f64(int q, const BatchBc* bcs, int nbc, long long nlinks, int parity, cudaStream_t st);
+#define ASLB_BATCH_CASE(Q, T)                                                                                      \
+  cudaError_t batch_step_q##Q##_##T(const BatchDom* doms, int ndom, const BatchWork& w, int links,                 \
+                                    const StepParams& p, int parity_in, int shape, cudaStream_t st);               \
+  cudaError_t batch_links_q##Q##_##T(const BatchBc* bcs, int nbc, long long nlinks, int parity, cudaStream_t st);
+ASLB_BATCH_CASE(15, f32)
+ASLB_BATCH_CASE(15, f16)
+ASLB_BATCH_CASE(15, f64)
+ASLB_BATCH_CASE(19, f32)
+ASLB_BATCH_CASE(19, f16)
+ASLB_BATCH_CASE(19, f64)
+ASLB_BATCH_CASE(27, f32)
+ASLB_BATCH_CASE(27, f16)
+ASLB_BATCH_CASE(27, f64)
+#undef ASLB_BATCH_CASE
+
+#define ASLB_BATCH_DISPATCH(what, ...)                                          \
+  switch (storage * 32 + q) {                                                   \
+    case ST_F32 * 32 + 15: return what##_q15_f32(__VA_ARGS__);                  \
+    case ST_F32 * 32 + 19: return what##_q19_f32(__VA_ARGS__);                  \
+    case ST_F32 * 32 + 27: return what##_q27_f32(__VA_ARGS__);                  \
+    case ST_F16 * 32 + 15: return what##_q15_f16(__VA_ARGS__);                  \
+    case ST_F16 * 32 + 19: return what##_q19_f16(__VA_ARGS__);                  \
+    case ST_F16 * 32 + 27: return what##_q27_f16(__VA_ARGS__);                  \
+    case ST_F64 * 32 + 15: return what##_q15_f64(__VA_ARGS__);                  \
+    case ST_F64 * 32 + 19: return what##_q19_f64(__VA_ARGS__);                  \
+    case ST_F64 * 32 + 27: return what##_q27_f64(__VA_ARGS__);                  \
+  }                                                                             \
+  return cudaErrorInvalidValue;
 
 int batch_shape_count() { return 5; }
 
@@ -41,24 +60,14 @@ void batch_work_tables(const std::vector<long long>& tile_cells, int sms, std::v
   }
 }
 
-cudaError_t launch_batch_step(int q, int storage, const BatchDom* doms, int ndom, const BatchWork& w, int fused,
+cudaError_t launch_batch_step(int q, int storage, const BatchDom* doms, int ndom, const BatchWork& w, int links,
                               const StepParams& p, int parity_in, int shape, cudaStream_t st) {
-  switch (storage) {
-    case ST_F32: return batch_step_f32(q, doms, ndom, w, fused, p, parity_in, shape, st);
-    case ST_F16: return batch_step_f16(q, doms, ndom, w, fused, p, parity_in, shape, st);
-    case ST_F64: return batch_step_f64(q, doms, ndom, w, fused, p, parity_in, shape, st);
-  }
-  return cudaErrorInvalidValue;
+  ASLB_BATCH_DISPATCH(batch_step, doms, ndom, w, links, p, parity_in, shape, st)
 }
 
 cudaError_t launch_batch_links(int q, int storage, const BatchBc* bcs, int nbc, long long nlinks, int parity,
                                cudaStream_t st) {
-  switch (storage) {
-    case ST_F32: return batch_links_f32(q, bcs, nbc, nlinks, parity, st);
-    case ST_F16: return batch_links_f16(q, bcs, nbc, nlinks, parity, st);
-    case ST_F64: return batch_links_f64(q, bcs, nbc, nlinks, parity, st);
-  }
-  return cudaErrorInvalidValue;
+  ASLB_BATCH_DISPATCH(batch_links, bcs, nbc, nlinks, parity, st)
 }
 
 }  // namespace aslb

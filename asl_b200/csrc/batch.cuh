@@ -29,11 +29,23 @@ __host__ __device__ constexpr int batch_shape_blocks(int shape) {
 __host__ __device__ constexpr bool batch_shape_pair(int shape) { return shape >= 3; }
 __host__ __device__ constexpr int batch_shape_threads(int shape) { return shape == 4 ? 320 : 256; }
 
-// A domain's fused-link words of a cell, from its one-word masks where it has
-// them; FP16 steps are bound by their instructions, not by their bytes, and
-// read the two words (48 channels: 0.263 ms per step, 0.276 with one word).
-template <int Q, class S>
+// A domain's fused-link words of a cell (LINKS: see BatchLinks). Where some
+// cell has both kinds of links, FP16 steps, bound by their instructions and not
+// by their bytes, read the two words (48 channels: 0.263 ms per step, 0.276
+// with the walls of the one-word form decoded).
+// Single: ms per step of channels, against the general form, in the fastest
+// shape: FP32 48 / 160 domains 0.362 / 1.143 (0.364 / 1.141), periodic 0.344 /
+// 1.093 (0.359 / 1.109); FP16 0.256 / 0.790 (0.261 / 0.806). It is not built
+// where it was slower: FP16 periodic 0.252 (0.243), FP64 0.631 (0.619), nor
+// for D3Q27, whose one-word masks never hold both kinds.
+template <int Q, class S, bool FLAT>
+constexpr bool kBatchSingle = Q != 27 && (sizeof(S) == 4 || (sizeof(S) == 2 && FLAT));
+template <int Q, class S, int LINKS>
 __device__ __forceinline__ uint2 batch_links(const BatchDom& D, unsigned s) {
+  if (LINKS == kLinksSingle) {
+    const uint32_t w = D.mask32[s];
+    return (w >> 31) ? make_uint2(0u, w & 0x7fffffffu) : make_uint2(w, 0u);
+  }
   if (sizeof(S) == 2) return D.mask[s];
   return D.mask32 ? link_words<Q>(D.mask32[s]) : D.mask[s];
 }
@@ -90,7 +102,7 @@ __device__ __forceinline__ int batch_domain(const BatchDom* __restrict__ doms, i
 // as one sequence of cells 256 at a time, so the next cell's link word is
 // fetched one step ahead across plane boundaries too and the domain's table
 // entry is read once per domain, not once per plane.
-template <int Q, class S, bool ODD, bool FUSED, bool FLAT, int BLOCKS>
+template <int Q, class S, bool ODD, int LINKS, bool FLAT, int BLOCKS>
 __global__ void __launch_bounds__(256, BLOCKS)
     k_batch_step(const BatchDom* __restrict__ doms, int ndom, const long long* __restrict__ starts, int K,
                  const StepParams p) {
@@ -114,7 +126,7 @@ __global__ void __launch_bounds__(256, BLOCKS)
     const unsigned nz = (unsigned)g.nz, nz_inv = D.nz_inv;
     S* F = (S*)D.F;
     const C om0 = std::is_same<C, double>::value ? C(D.om0d) : C(D.om0f);
-    const bool masked = FUSED && D.mask;
+    const bool masked = LINKS && D.mask;
     // storage index of cell l of plane x (y rows of nz cells, z fastest)
     auto cell_index = [&](int x, unsigned l, int& y, int& z) {
       unsigned yq = __umulhi(l + 1u, nz_inv);
@@ -133,7 +145,7 @@ __global__ void __launch_bounds__(256, BLOCKS)
     uint2 mnext = make_uint2(0u, 0u);
     if (masked && x <= xb) {
       int y1, z1;
-      mnext = batch_links<Q, S>(D, cell_index(x, l, y1, z1));
+      mnext = batch_links<Q, S, LINKS>(D, cell_index(x, l, y1, z1));
     }
     while (x <= xb) {
       int y, z;
@@ -147,13 +159,13 @@ __global__ void __launch_bounds__(256, BLOCKS)
       }
       if (masked && xn <= xb) {
         int y1, z1;
-        mnext = batch_links<Q, S>(D, cell_index(xn, ln, y1, z1));
+        mnext = batch_links<Q, S, LINKS>(D, cell_index(xn, ln, y1, z1));
       }
       int ox[3], oy[3], oz[3];
       batch_offsets<FLAT>(g, x, y, z, ox, oy, oz);
       C f[Q];
-      cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, s, ox, oy, oz, bounce, f);
-      batch_finish<Q, S, ODD, FUSED, FLAT>(F, g, p, (M*)D.rho, (M*)D.u, x, y, z, s, elide, f, om0);
+      cell_load<Q, S, ODD, LINKS != 0>(F, (unsigned)g.dstride, s, ox, oy, oz, bounce, f);
+      batch_finish<Q, S, ODD, LINKS != 0, FLAT>(F, g, p, (M*)D.rho, (M*)D.u, x, y, z, s, elide, f, om0);
       x = xn;
       l = ln;
     }
@@ -165,7 +177,7 @@ __global__ void __launch_bounds__(256, BLOCKS)
 // pair too is walked across plane boundaries: the planes of such batches hold
 // two to eight times NT cells, and stopping at each plane's end left a third
 // of the threads without a second cell.
-template <int Q, class S, bool ODD, bool FUSED, int BLOCKS, int NT>
+template <int Q, class S, bool ODD, int LINKS, int BLOCKS, int NT>
 __global__ void __launch_bounds__(NT, BLOCKS)
     k_batch_step_pair(const BatchDom* __restrict__ doms, int ndom, const long long* __restrict__ starts, int K,
                       const StepParams p) {
@@ -187,7 +199,7 @@ __global__ void __launch_bounds__(NT, BLOCKS)
     const unsigned plane_cells = (unsigned)(g.ny * g.nz);
     const unsigned nz = (unsigned)g.nz, nz_inv = D.nz_inv;
     S* F = (S*)D.F;
-    const bool masked = FUSED && D.mask;
+    const bool masked = LINKS && D.mask;
     const float om0 = D.om0f;
     auto row_of = [&](unsigned l, int& y, int& z) {
       unsigned yq = __umulhi(l + 1u, nz_inv);
@@ -215,8 +227,8 @@ __global__ void __launch_bounds__(NT, BLOCKS)
     advance(xb, lb, (unsigned)NT);
     uint2 na = make_uint2(0u, 0u), nb = make_uint2(0u, 0u);
     if (masked) {
-      if (xa <= x1) na = batch_links<Q, S>(D, cell_index(xa, la));
-      if (xb <= x1) nb = batch_links<Q, S>(D, cell_index(xb, lb));
+      if (xa <= x1) na = batch_links<Q, S, LINKS>(D, cell_index(xa, la));
+      if (xb <= x1) nb = batch_links<Q, S, LINKS>(D, cell_index(xb, lb));
     }
     while (xa <= x1) {
       const bool has_b = xb <= x1;
@@ -227,14 +239,14 @@ __global__ void __launch_bounds__(NT, BLOCKS)
       advance(xa, la, 2u * NT);
       advance(xb, lb, 2u * NT);
       if (masked) {
-        if (xa <= x1) na = batch_links<Q, S>(D, cell_index(xa, la));
-        if (xb <= x1) nb = batch_links<Q, S>(D, cell_index(xb, lb));
+        if (xa <= x1) na = batch_links<Q, S, LINKS>(D, cell_index(xa, la));
+        if (xb <= x1) nb = batch_links<Q, S, LINKS>(D, cell_index(xb, lb));
       }
       int ox[3], oy[3], oz[3];
       batch_offsets<true>(g, 0, 0, 0, ox, oy, oz);
       float fa[Q], fb[Q];
-      cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, sa, ox, oy, oz, ma.x, fa);
-      if (has_b) cell_load<Q, S, ODD, FUSED>(F, (unsigned)g.dstride, sb, ox, oy, oz, mb.x, fb);
+      cell_load<Q, S, ODD, LINKS != 0>(F, (unsigned)g.dstride, sa, ox, oy, oz, ma.x, fa);
+      if (has_b) cell_load<Q, S, ODD, LINKS != 0>(F, (unsigned)g.dstride, sb, ox, oy, oz, mb.x, fb);
       F2 f[Q], rho, u[3];
 #pragma unroll
       for (int i = 0; i < Q; ++i) f[i] = F2(fa[i], has_b ? fb[i] : 0.f);
@@ -262,8 +274,8 @@ __global__ void __launch_bounds__(NT, BLOCKS)
       }
       // store offsets recomputed after the collision (see batch_finish)
       const unsigned ds2 = after((unsigned)g.dstride, fa[0]);
-      cell_store<Q, S, ODD, FUSED>(F, p, ds2, after(sa, fa[0]), ox, oy, oz, ma.y, fa);
-      if (has_b) cell_store<Q, S, ODD, FUSED>(F, p, ds2, after(sb, fb[0]), ox, oy, oz, mb.y, fb);
+      cell_store<Q, S, ODD, LINKS != 0>(F, p, ds2, after(sa, fa[0]), ox, oy, oz, ma.y, fa);
+      if (has_b) cell_store<Q, S, ODD, LINKS != 0>(F, p, ds2, after(sb, fb[0]), ox, oy, oz, mb.y, fb);
     }
   }
 }
@@ -281,53 +293,57 @@ __global__ void __launch_bounds__(256)
   link_apply<Q, S>((S*)B.F, B.dstride, B.links, t < nlinks ? INT_MAX : 0, (int)(t - B.link0), B.ls, B.bp, parity);
 }
 
-template <int Q, class S, int SHAPE, bool FLAT>
-cudaError_t batch_step_shape(const BatchDom* doms, int ndom, const BatchWork& w, bool fused, const StepParams& p,
-                             int parity_in, cudaStream_t st) {
-  constexpr int BLOCKS = batch_shape_blocks(SHAPE);
+template <int Q, class S, int SHAPE, bool FLAT, int LINKS>
+cudaError_t batch_step_links(const BatchDom* doms, int ndom, const BatchWork& w, const StepParams& p, int parity_in,
+                             cudaStream_t st) {
+  constexpr int BLOCKS = batch_shape_blocks(SHAPE), NT = batch_shape_threads(SHAPE);
   const int grid = w.grid[BLOCKS - 2], K = w.group[BLOCKS - 2];
   const long long* starts = w.starts + w.off[BLOCKS - 2];
   const bool odd = parity_in == 0;
-  constexpr int NT = batch_shape_threads(SHAPE);
   auto go = [&](auto kern) { return launch_after(kern, grid, NT, 0, st, doms, ndom, starts, K, p); };
-  if constexpr (batch_shape_pair(SHAPE)) {
-    if (odd)
-      return fused ? go(k_batch_step_pair<Q, S, true, true, BLOCKS, NT>)
-                   : go(k_batch_step_pair<Q, S, true, false, BLOCKS, NT>);
-    return fused ? go(k_batch_step_pair<Q, S, false, true, BLOCKS, NT>)
-                 : go(k_batch_step_pair<Q, S, false, false, BLOCKS, NT>);
+  if constexpr (batch_shape_pair(SHAPE))
+    return odd ? go(k_batch_step_pair<Q, S, true, LINKS, BLOCKS, NT>) : go(k_batch_step_pair<Q, S, false, LINKS, BLOCKS, NT>);
+  else
+    return odd ? go(k_batch_step<Q, S, true, LINKS, FLAT, BLOCKS>) : go(k_batch_step<Q, S, false, LINKS, FLAT, BLOCKS>);
+}
+
+// Two cells per thread are built for D3Q15 / D3Q19 in 4- and 2-byte storage
+// without a periodic domain; other batches take the one-cell shape with the
+// same residency (in batches of periodic channels, two cells per thread with
+// the offsets wrapped were 6 to 20 % slower than one).
+template <int Q, class S, int SHAPE, bool FLAT>
+cudaError_t batch_step_shape(const BatchDom* doms, int ndom, const BatchWork& w, int links, const StepParams& p,
+                             int parity_in, cudaStream_t st) {
+  if constexpr (batch_shape_pair(SHAPE) && (!FLAT || Q == 27 || sizeof(S) == 8)) {
+    return batch_step_shape<Q, S, SHAPE == 3 ? 1 : 2, FLAT>(doms, ndom, w, links, p, parity_in, st);
   } else {
-    if (odd) return fused ? go(k_batch_step<Q, S, true, true, FLAT, BLOCKS>) : go(k_batch_step<Q, S, true, false, FLAT, BLOCKS>);
-    return fused ? go(k_batch_step<Q, S, false, true, FLAT, BLOCKS>) : go(k_batch_step<Q, S, false, false, FLAT, BLOCKS>);
+    if (links == kLinksNone) return batch_step_links<Q, S, SHAPE, FLAT, kLinksNone>(doms, ndom, w, p, parity_in, st);
+    if constexpr (kBatchSingle<Q, S, FLAT>)
+      if (links == kLinksSingle)
+        return batch_step_links<Q, S, SHAPE, FLAT, kLinksSingle>(doms, ndom, w, p, parity_in, st);
+    return batch_step_links<Q, S, SHAPE, FLAT, kLinksBoth>(doms, ndom, w, p, parity_in, st);
   }
 }
 
-// Two cells per thread are built for D3Q15 / D3Q19 in 4- and 2-byte storage;
-// other batches take the one-cell shape with the same residency. A batch with
-// a periodic domain has one shape (three blocks, two in FP64).
-template <int Q, class S, int SHAPE>
-cudaError_t batch_step_m(const BatchDom* doms, int ndom, const BatchWork& w, bool fused, const StepParams& p,
-                         int parity_in, cudaStream_t st) {
-  constexpr int ONE = SHAPE == 3 ? 1 : 2;
-  if constexpr (batch_shape_pair(SHAPE) && (Q == 27 || sizeof(S) == 8))
-    return batch_step_shape<Q, S, ONE, true>(doms, ndom, w, fused, p, parity_in, st);
-  else
-    return batch_step_shape<Q, S, SHAPE, true>(doms, ndom, w, fused, p, parity_in, st);
+template <int Q, class S, bool FLAT>
+cudaError_t batch_step_flat(const BatchDom* doms, int ndom, const BatchWork& w, int links, const StepParams& p,
+                            int parity_in, int shape, cudaStream_t st) {
+  switch (shape) {
+    case 0: return batch_step_shape<Q, S, 0, FLAT>(doms, ndom, w, links, p, parity_in, st);
+    case 1: return batch_step_shape<Q, S, 1, FLAT>(doms, ndom, w, links, p, parity_in, st);
+    case 2: return batch_step_shape<Q, S, 2, FLAT>(doms, ndom, w, links, p, parity_in, st);
+    case 3: return batch_step_shape<Q, S, 3, FLAT>(doms, ndom, w, links, p, parity_in, st);
+    case 4: return batch_step_shape<Q, S, 4, FLAT>(doms, ndom, w, links, p, parity_in, st);
+  }
+  return cudaErrorInvalidValue;
 }
 
 template <int Q, class S>
-cudaError_t batch_step_impl(const BatchDom* doms, int ndom, const BatchWork& w, int fused, const StepParams& p,
+cudaError_t batch_step_impl(const BatchDom* doms, int ndom, const BatchWork& w, int links, const StepParams& p,
                             int parity_in, int shape, cudaStream_t st) {
   if (w.ntiles <= 0) return cudaSuccess;
-  if (w.periodic) return batch_step_shape<Q, S, sizeof(S) == 8 ? 2 : 1, false>(doms, ndom, w, fused, p, parity_in, st);
-  switch (shape) {
-    case 0: return batch_step_m<Q, S, 0>(doms, ndom, w, fused, p, parity_in, st);
-    case 1: return batch_step_m<Q, S, 1>(doms, ndom, w, fused, p, parity_in, st);
-    case 2: return batch_step_m<Q, S, 2>(doms, ndom, w, fused, p, parity_in, st);
-    case 3: return batch_step_m<Q, S, 3>(doms, ndom, w, fused, p, parity_in, st);
-    case 4: return batch_step_m<Q, S, 4>(doms, ndom, w, fused, p, parity_in, st);
-  }
-  return cudaErrorInvalidValue;
+  return w.periodic ? batch_step_flat<Q, S, false>(doms, ndom, w, links, p, parity_in, shape, st)
+                    : batch_step_flat<Q, S, true>(doms, ndom, w, links, p, parity_in, shape, st);
 }
 
 template <int Q, class S>

@@ -142,10 +142,14 @@ struct BatchWork {
 // four blocks where that divides it).
 void batch_work_tables(const std::vector<long long>& tile_cells, int sms, std::vector<long long>& starts,
                        int (&grid)[3], int (&group)[3], long long (&off)[3]);
+// The fused links of a batch: none; of any kind; or every domain that has
+// links has them in one word per cell, and no cell has both kinds, so that the
+// word splits without looking at its walls.
+enum BatchLinks { kLinksNone = 0, kLinksBoth = 1, kLinksSingle = 2 };
 // One stream-collide step of every domain of a batch (same lattice, storage
 // and parity; CL_NONE), a persistent grid over all domains' tiles; `shape`
 // (0 .. batch_shape_count() - 1) picks the resident blocks per SM.
-cudaError_t launch_batch_step(int q, int storage, const BatchDom* doms, int ndom, const BatchWork& w, int fused,
+cudaError_t launch_batch_step(int q, int storage, const BatchDom* doms, int ndom, const BatchWork& w, int links,
                               const StepParams& p, int parity_in, int shape, cudaStream_t st);
 int batch_shape_count();
 // Every link of the entries (one condition position across the batch).

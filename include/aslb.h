@@ -422,10 +422,10 @@ long long aslb_batch_tiles(aslb_batch* b);
 /* Launch shape of the batched step: shape 0, 1, 2: one cell per thread at
  * 4, 3, 2 resident blocks of 256 threads per SM; 3, 4: two cells per thread
  * at 3 blocks of 256 or 2 of 320 threads (D3Q15 / D3Q19, FP32 / FP16, no
- * periodic domain; other batches take the one-cell shape of the same
- * residency). By default (or after shape -1) the first aslb_batch_run that
- * records a graph first times two real steps with every
- * shape and keeps the fastest (all shapes give identical results);
+ * periodic domain; other batches take shape 1 for 3 and shape 2 for 4). By
+ * default (or after shape -1) the first aslb_batch_run that records a graph
+ * first times two real steps with every shape and keeps the fastest (all
+ * shapes give identical results);
  * aslb_batch_shape_times returns those timings (ms, up to n; the count). */
 int aslb_batch_set_shape(aslb_batch* b, int shape);
 int aslb_batch_get_shape(aslb_batch* b);

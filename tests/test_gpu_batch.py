@@ -7,6 +7,7 @@ import pytest
 
 from asl_b200 import lbgk as A
 from asl_b200 import workloads as W
+from tests.test_gpu_parity import smooth_field, sphere_map
 
 pytestmark = pytest.mark.gpu
 
@@ -124,3 +125,50 @@ def test_batch_runs_across_domains_bitwise(gpu):
         assert batch.tiles > 4 * 148  # more tiles than blocks at every residency of a B200
         for w, lb, ref in zip(ws, lbs, refs):
             assert np.array_equal(lb.getF(), ref, equal_nan=True), (shape, w.name)
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16", "f64"])
+@pytest.mark.parametrize("q", [15, 19, 27])
+@pytest.mark.parametrize("mix", ["single", "both", "none"])
+@pytest.mark.parametrize("shape", [0, 1, 2, 3, 4])
+def test_batch_with_periodic_domains(gpu, storage, q, mix, shape):
+    """Periodic domains (x, z, all axes) beside walled ones, in every launch
+    shape, without links, with cells of one kind of link, and with cells of
+    both (a sphere cut by a fused wall): the domains stepped alone, both
+    parities."""
+    sizes = [((7, 5, 9), (0, 0, 0)), ((9, 8, 33), (1, 0, 0)), ((5, 9, 1), (0, 0, 1)), ((4, 6, 70), (0, 0, 1)),
+             ((6, 11, 32), (1, 1, 1)), ((2, 3, 65), (1, 0, 1))]
+    vt = {15: A.d3q15, 19: A.d3q19, 27: A.d3q27}[q]()
+
+    def domains():
+        out = []
+        for i, (size, per) in enumerate(sizes):
+            g = tuple(s + 2 for s in size)
+            lb = A.LBGK(A.Block(size), 0.01 + 0.01 * i, vt, storage=storage, periodic=tuple(bool(p) for p in per),
+                        body_force=(1e-4, 0, 1e-4), packed_rows=True)
+            A.LBGKUtilities(lb).initF(*smooth_field(g, i, amp=0.02))
+            walls = [w for w, p in zip((A.X0, A.XE, A.Y0, A.YE, A.Z0, A.ZE), np.repeat(per, 2)) if not p]
+            bcs = [A.generateBCNoSlip(lb, walls)] if walls and mix != "none" else []
+            if mix == "both" and size[1] == 8:  # through the wall y = 0
+                bcs.append(A.generateBCNoSlip(lb, sphere_map(g, (5.0, 0.5, 16.0), 2.7)))
+            elif mix != "none" and per == (1, 1, 1):
+                bcs.append(A.generateBCNoSlip(lb, sphere_map(g, (3.0, 6.0, 16.0), 2.4)))
+            for b in bcs:
+                b.fuse()
+            out.append((lb, bcs))
+        return out
+
+    alone, together = domains(), domains()
+    for lb, bcs in alone:
+        lb.run(5, bcs)
+        lb.sync()
+    batch = A.Batch([lb for lb, _ in together])
+    batch.setShape(shape)
+    batch.run(5, [bcs for _, bcs in together])
+    batch.sync()
+    assert batch.shape == shape
+    inner = (..., slice(1, -1), slice(1, -1), slice(1, -1))
+    for (a, _), (b, _) in zip(alone, together):
+        assert np.array_equal(a.getF(), b.getF(), equal_nan=True)
+        assert np.array_equal(a.getVelocity()[inner], b.getVelocity()[inner], equal_nan=True)
+        assert np.array_equal(a.getRho()[inner], b.getRho()[inner], equal_nan=True)
