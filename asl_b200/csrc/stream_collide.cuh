@@ -168,18 +168,6 @@ __device__ __forceinline__ void cell_store_flat(S* __restrict__ F, const StepPar
     store_slot<S>(F + (sl + (ODD ? p.slot[2][i] : p.slot[1][i])), f[i], MASKED && ((elide >> i) & 1u), p);
 }
 
-// Collision and wrap-aware stores of one cell (the batched step's form).
-template <int Q, class S, int CL, bool ODD, bool MASKED>
-__device__ __forceinline__ void cell_finish(S* __restrict__ F, const GridDesc& g, const StepParams& p,
-                                            typename MacroT<S>::T* __restrict__ rho_out,
-                                            typename MacroT<S>::T* __restrict__ u_out, int x, int y, int z,
-                                            unsigned s, const int (&ox)[3], const int (&oy)[3], const int (&oz)[3],
-                                            uint32_t elide, typename Store<S>::C (&f)[Q],
-                                            typename Store<S>::C om0) {
-  cell_collide<Q, S, CL>(g, p, rho_out, u_out, x, y, z, s, f, om0);
-  cell_store<Q, S, ODD, MASKED>(F, p, (unsigned)g.dstride, s, ox, oy, oz, elide, f);
-}
-
 // Whether any neighbour of a cell with coordinate v on a periodic axis of n
 // interior cells wraps to the opposite face.
 __device__ __forceinline__ bool wraps(int periodic_bit, int v, int n) { return periodic_bit && (v == 1 || v == n); }
@@ -320,7 +308,13 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, CL, FUSED>::blocks)
 // they are one sector per population, and cost a fully periodic 160^3 FP32
 // step 0.156 ms against 0.112). The plain step without links on a z axis that
 // does not wrap is faster with one cell per thread (384x192x192 FP32 0.376 ms
-// against 0.390).
+// against 0.390). Fused links on a z axis that wraps take one cell per thread
+// and z faces as single cells; the masked body has no wrapped offsets. (A porous
+// channel periodic in x and z, D3Q19 384x192x192, FP32 0.592 ms, FP16 0.467;
+// pairs that left both cells to the face blocks where either wraps took 0.751
+// and 0.638.)
+// One-word masks where every cell's links fit in one: FP16 D3Q19 porous channel
+// 320x208x256 0.357 ms with one word, 0.358 with two; D3Q15 0.319, 0.326.
 // A block walks `planes` consecutive x planes; each thread loads the
 // fused-link words of the next plane one iteration ahead, so that the
 // population loads, whose addresses those words select, do not wait for a
@@ -609,9 +603,10 @@ inline void step_launch_shape(const GridDesc& g, dim3& grid, dim3& block) {
 
 // x planes that a block walks: up to `most`, fewer where that would leave
 // SMs without a block (a small domain's step is one block's chain of planes).
+constexpr int kSms = 148;  // of a B200
 inline int planes_per_block(const GridDesc& g, const dim3& grid, int most) {
   int planes = most;
-  while (planes > 1 && (long long)grid.x * grid.y * ((g.nx + planes - 1) / planes) < 4 * 148) planes /= 2;
+  while (planes > 1 && (long long)grid.x * grid.y * ((g.nx + planes - 1) / planes) < 4 * kSms) planes /= 2;
   return planes;
 }
 

@@ -50,6 +50,31 @@ def test_pair_kernel_wraps_z_and_packs_bitwise(gpu, q, storage, closure, nz):
 
 
 @pytest.mark.parametrize("q", [15, 19, 27])
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("closure", [L.CLOSURE_NONE, L.CLOSURE_ASL_INTENT, L.CLOSURE_SMAGORINSKY])
+@pytest.mark.parametrize("nz", [1, 31, 33, 64, 97])
+@pytest.mark.parametrize("periodic", [(False, False, False), (True, True, False)])
+def test_closures_without_links_or_periodic_z(gpu, q, storage, closure, nz, periodic):
+    """The unmasked pair kernel (closures; FP16 as neighbouring cells) where z
+    does not wrap, its walls as separate conditions."""
+    shape = (5, 4, nz)
+    rho, u = smooth_field(tuple(s + 2 for s in shape), nz + q)
+
+    def make(variant):
+        lb = A.LBGK(A.Block(shape), 0.01, VT[q], storage=storage, periodic=periodic, body_force=(1e-4, -2e-4, 1e-4))
+        lb.setKernel(variant)
+        lb.setClosure(closure)
+        A.LBGKUtilities(lb).initF(rho, u)
+        walls = [A.generateBCNoSlip(lb, [A.Z0, A.ZE])]
+        if not periodic[0]:
+            walls.append(A.generateBCNoSlip(lb, [A.X0, A.XE, A.Y0, A.YE]))
+        lb.run(5, walls)
+        return lb
+
+    assert_same(populations(make))
+
+
+@pytest.mark.parametrize("q", [15, 19, 27])
 @pytest.mark.parametrize("storage", ["f32", "f16", "f64"])
 @pytest.mark.parametrize("nz", [5, 32, 40, 97])
 def test_fused_sphere_through_a_wall(gpu, q, storage, nz):
