@@ -257,6 +257,17 @@ inline FaceWork face_work(const GridDesc& g, bool paired, int threads, int gx, i
 // next plane's link words one iteration ahead (the population addresses
 // depend on them, so they must not cost a second memory round trip).
 constexpr int kOnePlanes = 4;
+// Where the kernel says that `planes` is at most kOnePlanes. The compiler then
+// orders the masked body's loads otherwise, for better or worse: 192x128x120
+// porous box, us per step, without / with: D3Q19 FP64 plain 184 / 171,
+// Smagorinsky 206 / 190, ASL's closure 190 / 204; D3Q19 FP32 learned 154 / 143,
+// plain 131 / 137; D3Q15 FP32 ASL's closure 120 / 111; D3Q27 FP32 ASL's closure
+// 217 / 200, Smagorinsky 199 / 210 (FP32: periodic in all axes).
+template <int Q, class S, int CL>
+constexpr bool kBoundPlanes = sizeof(S) == 8   ? Q == 19 && CL != CL_ASL_INTENT
+                              : Q == 15        ? sizeof(S) == 2 || CL != CL_NONE
+                              : Q == 19        ? CL == CL_MLP
+                                               : CL == CL_ASL_INTENT || (sizeof(S) == 2 && CL == CL_SMAGORINSKY);
 template <int Q, class S, int CL, bool ODD, bool FUSED>
 __global__ void __launch_bounds__(256, StepOccupancy<Q, S, CL, FUSED>::blocks)
     k_stream_collide(S* __restrict__ F, const __grid_constant__ GridDesc g, const __grid_constant__ StepParams p,
@@ -273,6 +284,7 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, CL, FUSED>::blocks)
   const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
   int x0 = (blockIdx.z - fw.fz) * planes + 1;
   int x1 = min(g.nx, x0 + planes - 1);
+  if (FUSED && kBoundPlanes<Q, S, CL>) x1 = min(x1, x0 + kOnePlanes - 1);
   if (z > g.nz || y > g.ny) return;
   // cells whose neighbours wrap across a periodic face belong to the face
   // kernel; skipped by the loop's range, the loop body has no branch
@@ -308,11 +320,12 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, CL, FUSED>::blocks)
 // they are one sector per population, and cost a fully periodic 160^3 FP32
 // step 0.156 ms against 0.112). The plain step without links on a z axis that
 // does not wrap is faster with one cell per thread (384x192x192 FP32 0.376 ms
-// against 0.390). Fused links on a z axis that wraps take one cell per thread
-// and z faces as single cells; the masked body has no wrapped offsets. (A porous
-// channel periodic in x and z, D3Q19 384x192x192, FP32 0.592 ms, FP16 0.467;
-// pairs that left both cells to the face blocks where either wraps took 0.751
-// and 0.638.)
+// against 0.390). Fused links on a z axis that wraps: the plain step of D3Q15 /
+// D3Q19 has a body with both (PZ), other steps take one cell per thread and z
+// faces as single cells (porous box periodic in all axes, D3Q19, us per step, PZ
+// / one cell / pairs left to the face blocks where either cell wraps: 192x128x120
+// FP32 102 / 131 / 182, FP16 75 / 94 / 123; 64x48x33 7.2 / 11.1 / 10.0, 7.2 /
+// 12.1 / 10.0).
 // One-word masks where every cell's links fit in one: FP16 D3Q19 porous channel
 // 320x208x256 0.357 ms with one word, 0.358 with two; D3Q15 0.319, 0.326.
 // A block walks `planes` consecutive x planes; each thread loads the
@@ -336,6 +349,27 @@ constexpr int kPairBlocks = Q == 27 ? (CL == CL_NONE || (ODD && !MASKED) ? 4 : 3
 // D3Q27 with links 0.198 / 0.206; with links FP16 D3Q19 0.362 / 0.355).
 template <int Q, int CL, bool MASKED>
 constexpr bool kPairPack = CL != CL_NONE || !MASKED || Q == 27;
+// Whether fused links take pairs. D3Q27's two cells leave too few registers in
+// FP16 (more instructions per byte) and with the learned closure: 192x128x120
+// porous box, us per step, pairs / one cell: FP16 plain 110 / 104, ASL's closure
+// 132 / 114, Smagorinsky 133 / 117, learned 134 / 118; FP32 learned 204 / 154,
+// but plain 140 / 144 and ASL's closure 155 / 168.
+template <int Q, class S, int CL>
+constexpr bool kPairLinks = Q != 27 || (sizeof(S) == 4 && CL != CL_MLP);
+// Whether the body with links also wraps z (PZ).
+template <int Q, int CL>
+constexpr bool kPairWraps = Q != 27 && CL == CL_NONE;
+// Whether a domain's step takes pairs. D3Q27 in FP32 where z does not wrap: the
+// learned closure without links 140 / 132; Smagorinsky 158 / 150 with links and
+// 128 / 125 without, but in rows that fill the lanes' 64 cells 209 / 211 and
+// 175 / 176 (256x128x128).
+template <int Q, class S, int CL>
+inline bool takes_pairs(const GridDesc& g, bool fused) {
+  const bool pz = g.periodic & 4;
+  if (fused ? !kPairLinks<Q, S, CL> || (pz && !kPairWraps<Q, CL>) : !pz && CL == CL_NONE) return false;
+  if (Q == 27 && !pz && (CL == CL_MLP || (CL == CL_SMAGORINSKY && g.nz % 64 != 0))) return false;
+  return true;
+}
 
 // Offsets of a cell and of the cells below and above it along z: the slots at
 // c_z = 0, at z - 1 and at z + 1, wrapped on a periodic z axis.
@@ -354,7 +388,7 @@ __device__ __forceinline__ ZBase z_base(const GridDesc& g, unsigned s, int z) {
 }
 __device__ __forceinline__ unsigned z_pick(const ZBase& b, int dz) { return dz == 0 ? b.at : (dz < 0 ? b.below : b.above); }
 
-template <int Q, class S, bool ODD, bool MASKED>
+template <int Q, class S, bool ODD, bool MASKED, bool PZ>
 __device__ __forceinline__ void pair_load(const S* __restrict__ F, const ZBase& b, const StepParams& p, uint32_t bounce,
                                           float (&f)[Q]) {
   using Lt = Lattice<Q>;
@@ -364,20 +398,21 @@ __device__ __forceinline__ void pair_load(const S* __restrict__ F, const ZBase& 
     if (MASKED) {
       // ODD: pull, or the opposite own slot when bounced; EVEN: the reverse
       const bool bb = (bounce >> i) & 1u;
-      at = b.at + ((ODD != bb) ? p.slot[0][i] : p.slot[3][i]);
+      const unsigned pull = (PZ ? z_pick(b, -Lt::c(i, 2)) : b.at) + p.slot[0][i];
+      at = (ODD != bb) ? pull : b.at + p.slot[3][i];
     } else {
       at = ODD ? z_pick(b, -Lt::c(i, 2)) + p.slot[0][i] : b.at + p.slot[3][i];
     }
     f[i] = Store<S>::load_c(F + at);
   }
 }
-template <int Q, class S, bool ODD, bool MASKED>
+template <int Q, class S, bool ODD, bool MASKED, bool PZ>
 __device__ __forceinline__ void pair_store(S* __restrict__ F, const ZBase& b0, const StepParams& p, uint32_t elide,
                                            const float (&f)[Q]) {
   using Lt = Lattice<Q>;
   ZBase b = b0;
   b.at = after(b.at, f[0]);
-  if (!MASKED) {
+  if (!MASKED || PZ) {
     b.below = after(b.below, f[0]);
     b.above = after(b.above, f[0]);
   } else {
@@ -392,22 +427,22 @@ __device__ __forceinline__ void pair_store(S* __restrict__ F, const ZBase& b0, c
 
 // One pair: cells (x, y, za) and, with has_b, (x, y, za + 32) at storage
 // indices sa and sa + 32, with their (bounce, elide) words.
-template <int Q, class S, int CL, bool ODD, bool MASKED>
+template <int Q, class S, int CL, bool ODD, bool MASKED, bool PZ>
 __device__ __forceinline__ void pair_step(S* __restrict__ F, const GridDesc& g, const StepParams& p, int x, int y,
                                           int za, bool has_b, unsigned sa, uint2 ma, uint2 mb,
                                           float* __restrict__ rho_out, float* __restrict__ u_out) {
   const unsigned sb = sa + 32u;
   const int zb = za + 32;
-  const ZBase ba = z_base<!MASKED>(g, sa, za), bb = z_base<!MASKED>(g, sb, zb);
+  const ZBase ba = z_base<!MASKED || PZ>(g, sa, za), bb = z_base<!MASKED || PZ>(g, sb, zb);
   float fa[Q], fb[Q];
-  pair_load<Q, S, ODD, MASKED>(F, ba, p, ma.x, fa);
-  if (has_b) pair_load<Q, S, ODD, MASKED>(F, bb, p, mb.x, fb);
+  pair_load<Q, S, ODD, MASKED, PZ>(F, ba, p, ma.x, fa);
+  if (has_b) pair_load<Q, S, ODD, MASKED, PZ>(F, bb, p, mb.x, fb);
   if constexpr (!kPairPack<Q, CL, MASKED>) {
     cell_collide<Q, S, CL>(g, p, rho_out, u_out, x, y, za, sa, fa, p.om0f);
-    pair_store<Q, S, ODD, MASKED>(F, ba, p, ma.y, fa);
+    pair_store<Q, S, ODD, MASKED, PZ>(F, ba, p, ma.y, fa);
     if (has_b) {
       cell_collide<Q, S, CL>(g, p, rho_out, u_out, x, y, zb, sb, fb, p.om0f);
-      pair_store<Q, S, ODD, MASKED>(F, bb, p, mb.y, fb);
+      pair_store<Q, S, ODD, MASKED, PZ>(F, bb, p, mb.y, fb);
     }
   } else {
     F2 f[Q], rho, u[3], cs2 = F2(0.f);
@@ -433,14 +468,15 @@ __device__ __forceinline__ void pair_step(S* __restrict__ F, const GridDesc& g, 
       fa[i] = f[i].lo();
       fb[i] = f[i].hi();
     }
-    pair_store<Q, S, ODD, MASKED>(F, ba, p, ma.y, fa);
-    if (has_b) pair_store<Q, S, ODD, MASKED>(F, bb, p, mb.y, fb);
+    pair_store<Q, S, ODD, MASKED, PZ>(F, ba, p, ma.y, fa);
+    if (has_b) pair_store<Q, S, ODD, MASKED, PZ>(F, bb, p, mb.y, fb);
   }
 }
 
-// FUSED: 0 no links, 1 the two-word masks, 2 the one-word masks.
-template <int Q, class S, int CL, bool ODD, int FUSED>
-__global__ void __launch_bounds__(kPairThreads, kPairBlocks<Q, CL, FUSED != 0, ODD>)
+// FUSED: 0 no links, 1 the two-word masks, 2 the one-word masks. PZ: with links,
+// the z axis wraps (three bases per cell: five blocks instead of six).
+template <int Q, class S, int CL, bool ODD, int FUSED, bool PZ = false>
+__global__ void __launch_bounds__(kPairThreads, kPairBlocks<Q, CL, FUSED != 0 && !PZ, ODD>)
     k_step_pair(S* __restrict__ F, const __grid_constant__ GridDesc g, const __grid_constant__ StepParams p,
                 const __grid_constant__ FaceWork fw, int planes, float* __restrict__ rho_out,
                 float* __restrict__ u_out) {
@@ -486,9 +522,9 @@ __global__ void __launch_bounds__(kPairThreads, kPairBlocks<Q, CL, FUSED != 0, O
     // D3Q27 (the closures' and its own registers leave room for both bodies):
     // 64 cells without a link take the body without selects
     if (FUSED && (Q != 27 || __any_sync(__activemask(), wa.x | wa.y | wb.x | wb.y)))
-      pair_step<Q, S, CL, ODD, true>(F, g, p, x, y, za, has_b, sa, split(wa), split(wb), rho_out, u_out);
+      pair_step<Q, S, CL, ODD, true, PZ>(F, g, p, x, y, za, has_b, sa, split(wa), split(wb), rho_out, u_out);
     else
-      pair_step<Q, S, CL, ODD, false>(F, g, p, x, y, za, has_b, sa, make_uint2(0u, 0u), make_uint2(0u, 0u), rho_out,
+      pair_step<Q, S, CL, ODD, false, PZ>(F, g, p, x, y, za, has_b, sa, make_uint2(0u, 0u), make_uint2(0u, 0u), rho_out,
                                       u_out);
     wa = na;
     wb = nb;
@@ -654,17 +690,22 @@ cudaError_t step_q_s_cl(const DomainDev& d, const StepParams& p, int parity_in, 
     }
   }
   if constexpr (!std::is_same<S, double>::value) {
-    // two cells per thread: see k_step_pair
-    const bool pz = d.g.periodic & 4;
-    if (d.variant == 0 && (fused ? !pz : (pz || CL != CL_NONE))) {
+    if (d.variant == 0 && takes_pairs<Q, S, CL>(d.g, fused)) {
       const int planes = pair_launch_shape(d.g, grid, block);
       const FaceWork fw = face_work(d.g, true, block.x * block.y, grid.x, grid.y);
       grid.z += fw.fz;
       auto go = [&](auto kern) { return launch_after(kern, grid, block, 0, st, F, d.g, p, fw, planes, rho, u); };
       const bool odd = parity_in == 0;
       if (!fused) return odd ? go(k_step_pair<Q, S, CL, true, 0>) : go(k_step_pair<Q, S, CL, false, 0>);
-      if (!p.mask32) return odd ? go(k_step_pair<Q, S, CL, true, 1>) : go(k_step_pair<Q, S, CL, false, 1>);
-      return odd ? go(k_step_pair<Q, S, CL, true, 2>) : go(k_step_pair<Q, S, CL, false, 2>);
+      if constexpr (kPairWraps<Q, CL>)
+        if (d.g.periodic & 4) {
+          if (!p.mask32) return odd ? go(k_step_pair<Q, S, CL, true, 1, true>) : go(k_step_pair<Q, S, CL, false, 1, true>);
+          return odd ? go(k_step_pair<Q, S, CL, true, 2, true>) : go(k_step_pair<Q, S, CL, false, 2, true>);
+        }
+      if constexpr (kPairLinks<Q, S, CL>) {
+        if (!p.mask32) return odd ? go(k_step_pair<Q, S, CL, true, 1>) : go(k_step_pair<Q, S, CL, false, 1>);
+        return odd ? go(k_step_pair<Q, S, CL, true, 2>) : go(k_step_pair<Q, S, CL, false, 2>);
+      }
     }
   }
   const int planes = plane_launch_shape(d.g, grid, block);
