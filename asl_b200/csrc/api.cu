@@ -88,9 +88,9 @@ struct aslb_lbgk {
   std::vector<LinkGroup> groups;
   std::vector<aslb_bc*> groups_key;
   // the condition list of the last run, how many runs and steps in a row have
-  // had it, and the steps from which another check is worth it
+  // had it, and the steps from which to merge it (-1: not known yet)
   std::vector<aslb_bc*> run_key;
-  long long run_count = 0, run_steps = 0, run_try = 0;
+  long long run_count = 0, run_steps = 0, run_need = -1;
   // fused no-slip conditions
   // fresh: populations were (re)initialised and no fused condition has run
   // since, so incoming slots still hold their initial values and the next
@@ -827,15 +827,16 @@ namespace {
 // entry: 25 us for the four walls, inlet and outlet of a 128x64x64 channel
 // (204,288 links), 2.1 ms with the 254,883 links of a porous map in it, where
 // merging saves 5 us per step. So a list is checked once its steps in a row
-// would have paid for the walk (kGroupWalk entries per step and launch saved),
-// and takes the place of another list's launches only in its second run in a
-// row or in a long one: a program that alternates between lists keeps the
-// launches of the first (64x32x32 porous channel, two lists in turn, runs of
-// four steps: 0.34 ms per pair of runs, 0.98 when every run merged its own).
+// are a quarter of what pays for the walk (kGroupWalk entries per step and launch
+// saved; the walk's length is known from the ends of the overlaps, 10 us), and
+// takes the place of another list's launches only in its second run in a row or
+// in a long one: a program that alternates between lists keeps the launches of
+// the first (64x32x32 porous channel, two lists in turn, runs of four steps:
+// 0.34 ms per pair of runs, 0.98 when every run merged its own).
 constexpr long long kGroupLinks = 1 << 20;
 constexpr size_t kGroupDropped = 16384;
 constexpr int kGroupSteps = 4, kGroupLongRun = 32;
-constexpr long long kGroupWalk = 1000;
+constexpr long long kGroupWalk = 4000;
 
 struct LinkRange {  // ascending storage indices, all displaced by off
   const int* p;
@@ -852,11 +853,10 @@ LinkRange outgoing(const aslb_bc* b, int k) {  // direction inv k at the fluid e
 }
 // Calls f(index in a, index in b) for every common index of two ranges until f
 // returns true; true then. Only the part of each range inside the other's is
-// walked (a wall's links lie in one plane of a channel), and what is walked is
-// taken off `walk`; below zero nothing is walked any more and the answer means
-// nothing.
+// walked (a wall's links lie in one plane of a channel); with `count` nothing is
+// walked, and what would be is added to it.
 template <class F>
-bool common(const LinkRange& a, const LinkRange& b, long long& walk, F f) {
+bool common(const LinkRange& a, const LinkRange& b, long long* count, F f) {
   if (a.p == a.e || b.p == b.e) return false;
   const int lo = std::max(a.p[0] + a.off, b.p[0] + b.off), hi = std::min(a.e[-1] + a.off, b.e[-1] + b.off);
   if (lo > hi) return false;
@@ -864,8 +864,10 @@ bool common(const LinkRange& a, const LinkRange& b, long long& walk, F f) {
   const int* j = std::lower_bound(b.p, b.e, lo - b.off);
   const int* ie = std::upper_bound(i, a.e, hi - a.off);
   const int* je = std::upper_bound(j, b.e, hi - b.off);
-  walk -= (ie - i) + (je - j);
-  if (walk < 0) return false;
+  if (count) {
+    *count += (ie - i) + (je - j);
+    return false;
+  }
   while (i != ie && j != je) {
     const int d = (*i + a.off) - (*j + b.off);
     if (d == 0 && f(i - a.p, j - b.p)) return true;
@@ -874,11 +876,11 @@ bool common(const LinkRange& a, const LinkRange& b, long long& walk, F f) {
   }
   return false;
 }
-bool conflict(const aslb_bc* a, const aslb_bc* b, int q, long long& walk) {
+bool conflict(const aslb_bc* a, const aslb_bc* b, int q, long long* count) {
   auto yes = [](long long, long long) { return true; };
   for (int k = 1; k < q; ++k) {
     const int j = a->ls.inv[k];
-    if (common(outgoing(a, k), incoming(b, j), walk, yes) || common(incoming(a, j), outgoing(b, k), walk, yes)) return true;
+    if (common(outgoing(a, k), incoming(b, j), count, yes) || common(incoming(a, j), outgoing(b, k), count, yes)) return true;
   }
   return false;
 }
@@ -901,9 +903,9 @@ cudaError_t mark_dropped(aslb_lbgk* h, aslb_bc* bc, const std::vector<int>& drop
   return e;
 }
 
-// The merged launches of a condition list. Gives up (false) when the check
-// walks more than `walk` list entries; sets nothing on the device.
-bool find_groups(const aslb_lbgk* h, const std::vector<aslb_bc*>& key, long long walk, std::vector<LinkGroup>& out) {
+// The merged launches of a condition list; sets nothing on the device. With
+// `count` only the list entries that the check would walk (`out` means nothing).
+void find_groups(const aslb_lbgk* h, const std::vector<aslb_bc*>& key, long long* count, std::vector<LinkGroup>& out) {
   const int q = h->d.q;
   // a condition that stands in the list more than once keeps its own launches:
   // which of its links a later condition writes differs from place to place,
@@ -917,7 +919,7 @@ bool find_groups(const aslb_lbgk* h, const std::vector<aslb_bc*>& key, long long
     size_t j = i, dropped = 0;
     for (; j < key.size() && plain(key[j]) && (long long)links + key[j]->nd <= kGroupLinks; ++j) {
       bool ok = key[j]->bp.scale == key[i]->bp.scale;
-      for (size_t m = i; ok && m < j; ++m) ok = !conflict(key[m], key[j], q, walk);
+      for (size_t m = i; ok && m < j; ++m) ok = !conflict(key[m], key[j], q, count);
       int used = 0;
       for (int k = 1; k < q; ++k) used += key[j]->ls.seg[k + 1] > key[j]->ls.seg[k];
       if (!ok || g.segs.n + used > kLinkSegs) break;
@@ -937,7 +939,7 @@ bool find_groups(const aslb_lbgk* h, const std::vector<aslb_bc*>& key, long long
         g.segs.vald[s] = b->ls.vald[k];
         // links that this condition writes after an earlier one
         for (size_t m = 0; m < g.bcs.size(); ++m)
-          common(incoming(g.bcs[m], k), incoming(b, k), walk, [&](long long x, long long) {
+          common(incoming(g.bcs[m], k), incoming(b, k), count, [&](long long x, long long) {
             g.dropped[m].push_back(g.bcs[m]->ls.seg[k] + (int)x);
             ++dropped;
             return false;
@@ -947,7 +949,6 @@ bool find_groups(const aslb_lbgk* h, const std::vector<aslb_bc*>& key, long long
       g.bcs.push_back(b);
       g.dropped.emplace_back();
     }
-    if (walk < 0) return false;
     if (g.bcs.size() < 2 || dropped > kGroupDropped) {
       ++i;
       continue;
@@ -956,7 +957,6 @@ bool find_groups(const aslb_lbgk* h, const std::vector<aslb_bc*>& key, long long
     out.push_back(g);
     i = j;
   }
-  return true;
 }
 
 // Called by every run that is not recorded, before its first step: counts the
@@ -964,18 +964,23 @@ bool find_groups(const aslb_lbgk* h, const std::vector<aslb_bc*>& key, long long
 int update_groups(aslb_lbgk* h, const std::vector<aslb_bc*>& key, int nsteps) {
   if (h->run_key != key) {
     h->run_key = key;
-    h->run_count = h->run_steps = h->run_try = 0;
+    h->run_count = h->run_steps = 0;
+    h->run_need = -1;
   }
   h->run_count += 1;
   h->run_steps += nsteps;
-  if (key.size() < 2 || nsteps < kGroupSteps || h->groups_key == key || h->run_steps < h->run_try) return ASLB_OK;
+  if (key.size() < 2 || nsteps < kGroupSteps || h->groups_key == key || h->run_steps < h->run_need) return ASLB_OK;
   if (!h->groups.empty() && h->run_count < 2 && nsteps < kGroupLongRun) return ASLB_OK;
   std::vector<LinkGroup> found;
-  if (!find_groups(h, key, h->run_steps * kGroupWalk * (long long)(key.size() - 1), found)) {
-    h->run_try = 2 * h->run_steps;
-    return ASLB_OK;
+  if (h->run_need < 0) {
+    long long entries = 0;
+    find_groups(h, key, &entries, found);
+    found.clear();
+    h->run_need = entries / (kGroupWalk * (long long)(key.size() - 1));
+    if (h->run_steps < h->run_need) return ASLB_OK;
   }
-  h->run_try = LLONG_MAX;  // found for good, or there are none
+  find_groups(h, key, nullptr, found);
+  h->run_need = LLONG_MAX;  // found for good, or there are none
   if (found.empty()) return ASLB_OK;
   drop_graph(h);  // it may hold merged launches
   for (LinkGroup& g : found)
